@@ -310,7 +310,7 @@ agx_status agx_scenario_create(const agx_mesh_desc* m, const agx_params* p, agx_
   if (enqueue_order_init(s, s->stream) != cudaSuccess) return fin(fail(AGX_E_CUDA, "order init failed"));
   const size_t N = s->N, B = s->B, E = s->E;
   struct Up { const void* src; const void* dst; size_t bytes; } ups[] = {
-      {m->conn, s->d.conn, N * 16}, {m->surr, s->d.surr, N * 16}, {m->geo, s->d.geo, N * GEO_STRIDE * 8},
+      {m->conn, s->d.conn, N * 16}, {m->surr, s->d.surr, N * 16}, {m->geo, s->d.sl0, N * GEO_STRIDE * 8},
       {m->edge_slot, s->d.edge_slot, E * 4}, {m->edge_opp, s->d.edge_opp, E * 4},
       {m->normals, s->d.normals, N * 48}, {m->edgelengths, s->d.lengths, N * 24},
       {m->radii, s->d.radii, N * 8}, {m->areas, s->d.areas, N * 8}, {m->inv_area, s->d.inv_area, N * 8},
@@ -321,6 +321,10 @@ agx_status agx_scenario_create(const agx_mesh_desc* m, const agx_params* p, agx_
     if (cudaMemcpyAsync((void*)u.dst, u.src, u.bytes, cudaMemcpyHostToDevice, s->stream) != cudaSuccess)
       return fin(fail(AGX_E_CUDA, "table upload failed"));
   }
+  // the geometry rows went to the slot arrays (18 doubles a cell, not in use
+  // yet), which are cleared again once the rows are transposed
+  if (enqueue_geo_transpose(s, s->stream, s->d.sl0) != cudaSuccess) return fin(fail(AGX_E_CUDA, "geometry transposition failed"));
+  if (cudaMemsetAsync(s->d.sl0, 0, N * GEO_STRIDE * 8, s->stream) != cudaSuccess) return fin(fail(AGX_E_CUDA, "memset failed"));
   init_clock(s->clock_host, *p);
   if ((st = push_clock(s)) != AGX_OK) return fin(st);
   return AGX_OK;

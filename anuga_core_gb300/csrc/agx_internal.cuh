@@ -159,7 +159,7 @@ struct Dev {
   Params P;
   const int4* conn;
   const int4* surr;
-  const double* geo;
+  const double* geo;                     // [GEO_STRIDE][N]
   const int* edge_slot;
   const int* edge_opp;
   const double* normals;
@@ -271,5 +271,6 @@ cudaError_t enqueue_saxpy(Scenario* s, cudaStream_t st, double a, double b);
 cudaError_t enqueue_divide(Scenario* s, cudaStream_t st, double divisor);
 cudaError_t enqueue_reset_accum(Scenario* s, cudaStream_t st);
 cudaError_t enqueue_order_init(Scenario* s, cudaStream_t st);
+cudaError_t enqueue_geo_transpose(Scenario* s, cudaStream_t st, const double* rows);
 
 }  // namespace agx

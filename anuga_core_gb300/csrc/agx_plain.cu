@@ -18,37 +18,17 @@
 namespace agx {
 
 constexpr int TPB = 256;
-// resident blocks of TPB threads per SM asked of the compiler for the
-// extrapolation, flux and accumulation kernels (register budgets): four
-// blocks (64 registers) for the extrapolation and the flux, measured faster
-// on the 4.0M-triangle DE1 step (extrapolation in class order 2.49 -> 2.39 ms,
-// flux 1.757 -> 1.714 ms); the accumulation keeps its own budget
+// resident blocks per SM asked of the compiler for the extrapolation, flux
+// and accumulation kernels (register budgets): 64 registers for the
+// extrapolation and the flux; the accumulation keeps its own budget
 #ifndef AGX_MINB_EXTRAP
-#define AGX_MINB_EXTRAP 4
+#define AGX_MINB_EXTRAP 8
 #endif
 #ifndef AGX_MINB_FLUX
 #define AGX_MINB_FLUX 4
 #endif
 #ifndef AGX_MINB_ACCUM
 #define AGX_MINB_ACCUM 1
-#endif
-// 1: the step's extrapolations visit the cells grouped by the branches each
-// took in the previous extrapolation (per-cell results do not depend on the
-// order in which cells are visited).  Measured on the 4.0M-triangle DE1 step:
-// extrapolation 2.76 -> 2.31 ms, step 6.53 -> 6.12 ms with the sort once per
-// step on the dry and wet/dry-factor classes.
-#ifndef AGX_EXTRAP_ORDER
-#define AGX_EXTRAP_ORDER 1
-#endif
-// the class bits the sort distinguishes (see k_extrap): 2 = dry cell and
-// wet/dry factor below 1
-#ifndef AGX_CLASS_BITS
-#define AGX_CLASS_BITS 2
-#endif
-// 1: the cells are sorted after every extrapolation of a step; 2: only after
-// its last (the step's stages visit the cells in one order)
-#ifndef AGX_SORT_CADENCE
-#define AGX_SORT_CADENCE 2
 #endif
 static const double kNaN = __builtin_nan("");
 
@@ -116,61 +96,135 @@ __global__ void k_prep(Dev d, int mode) {
   }
 }
 
-// ORD: thread i takes cell order[i] and records the cell's branch class
+// Extrapolation (:1418-1896): a block takes XCELLS cells, one per lane, and
+// each of its four warps reconstructs one quantity of them (stage, depth, x
+// and y velocity).  The height warp forms the wet/dry factor the others'
+// limiters need while they form their jumps, and hands over its edge depths
+// for the bed (w - h) and the momenta (u h).  The FP64 pipe bounds it on large
+// meshes (per launch of a 4.0M-triangle DE1 step 1.00 -> 0.98 ms against one
+// thread per cell) and the chain of one thread's operations on small ones,
+// which is a quarter as long this way: 26 -> 7.4 us on 396 cells, 41 -> 26 us
+// on 40,000 (DE0), 96 -> 70 us on 250,000 (DE1).
+// ORD: lane i takes cell order[i] and the height warp records its branch class.
+constexpr int XCELLS = 32;
+constexpr int XTPB = 4 * XCELLS;
 template <bool VERT, bool ORD = false>
-__global__ void __launch_bounds__(TPB, AGX_MINB_EXTRAP) k_extrap(Dev d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= d.N) return;
-  const int k = ORD ? d.order[i] : i;
-  EdgeOut E;
-  int cls = 0;
-  const bool sdry = extrap_cell(d.P, k, d.conn, d.surr, d.geo, d.w, d.h, d.u, d.v, E, ORD ? &cls : nullptr);
-  if (ORD) {
-    // the classes the sort distinguishes: all eight bits, or the four
-    // limiter bits merged into one (5), or none of them (4), or only the
-    // dry and wet/dry-factor bits (2), or only the dry bit (1).  Measured
-    // extrapolation per 4.0M-triangle DE1 step: 2.38, 2.39, 2.31, 2.31,
-    // 2.73 ms (2.76 unsorted): what pays is keeping the cells of the wet/dry
-    // fronts (factor below 1: the divided-out factor, mixed betas, limiter
-    // products) out of the warps of the rest; finer classes only cut the
-    // cells' runs shorter.
-    if (AGX_CLASS_BITS == 5) cls = (cls & 15) | ((cls & 240) ? 16 : 0);
-    if (AGX_CLASS_BITS == 4) cls &= 15;
-    if (AGX_CLASS_BITS == 2) cls &= 12;
-    if (AGX_CLASS_BITS == 1) cls &= 4;
-    d.cls[k] = (unsigned char)cls;
-  }
-  const size_t b = 3 * (size_t)k;
+__global__ void __launch_bounds__(XTPB, AGX_MINB_EXTRAP) k_extrap(Dev d) {
+  __shared__ double s_factor[XCELLS];
+  __shared__ double s_h[3][XCELLS];
+  const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+  const int at = blockIdx.x * XCELLS + lane;
+  const bool in = at < d.N;
+  const int k = ORD ? d.order[in ? at : d.N - 1] : (in ? at : d.N - 1);
+  const Params& P = d.P;
+  const int4 s = d.surr[k];
+  const int meta = d.conn[k].w;
+  const int nb = meta_nb(meta);
+  const double* A = q == 0 ? d.w : q == 1 ? d.h : q == 2 ? d.u : d.v;
+  const double beta0 = q < 2 ? P.beta_w : q == 2 ? P.beta_uh : P.beta_vh;
+  const double beta0_dry = q < 2 ? P.beta_w_dry : q == 2 ? P.beta_uh_dry : P.beta_vh_dry;
+  double qc = A[k], q0 = A[s.x], q1 = A[s.y], q2 = A[s.z];
+  const double hk = d.h[k], h0 = d.h[s.x], h1 = d.h[s.y], h2 = d.h[s.z];
+  const bool sdry = (dlt(h0, P.hmin) | (s.x == k)) & (dlt(h1, P.hmin) | (s.y == k)) & (dlt(h2, P.hmin) | (s.z == k));
+  const bool dry = dlt(hk, P.hmin);
+  if (q >= 2) {
+    if (sdry) qc = 0.0;
+    // Neighbour velocities can be stale-zeroed only for a dry cell (a wet
+    // neighbour rules out "surrounded by dry"); they matter only if the dry
+    // reconstruction has a positive beta (the factor of a dry cell is 0), or
+    // towards the one neighbour of a cell with two boundary edges.
+    if (nb == 2 || (nb <= 1 && dry && (dgt0(P.beta_uh_dry) || dgt0(P.beta_vh_dry)))) {
+      const int sv[3] = {s.x, s.y, s.z};
+      double* qv[3] = {&q0, &q1, &q2};
 #pragma unroll
-  for (int i = 0; i < 3; i++) {
-    d.we[b + i] = E.w[i];
-    d.he[b + i] = E.h[i];
-    d.uhe[b + i] = E.uh[i];
-    d.vhe[b + i] = E.vh[i];
-    d.ze[b + i] = E.z[i];
+      for (int i = 0; i < 3; i++) {
+        double us, vs;
+        if (sv[i] != k) {
+          neighbour_uv(P, sv[i], meta_before(meta, i) != 0, d.surr, d.h, d.u, d.v, us, vs);
+          *qv[i] = q == 2 ? us : vs;
+        }
+      }
+    }
+    if (s.x == k) q0 = qc;
+    if (s.y == k) q1 = qc;
+    if (s.z == k) q2 = qc;
   }
-  if (sdry) {
-    d.uh[k] = 0.0;
-    d.vh[k] = 0.0;
+  // The factor is 0 where a depth around the cell is at most hmin (its third
+  // term is 0 over a positive number): with a dry beta of 0 the edges then
+  // take the cell's value and no gradient is needed.
+  const double hlo = dmin(dmin(h0, dmin(h1, h2)), hk);
+  const bool factor0 = dgt0(P.hmin) && dle(hlo, P.hmin);
+  const bool grad = nb <= 1 && (dgt0(beta0_dry) || (dgt0(beta0) && !factor0));
+  double G[GEO_STRIDE];
+  double jump[3], lo = 0.0, hi = 0.0, E[3];
+  if (grad || nb == 2) {
+#pragma unroll
+    for (int i = 0; i < GEO_STRIDE; i++) G[i] = d.geo[(size_t)i * d.N + k];
   }
-  if (!VERT && d.P.sloped_mannings) {
-    double vx[3];
-    vertex_from_edges(E.z, vx);   // sloped friction reads the bed vertex values
-    for (int i = 0; i < 3; i++) d.zv[b + i] = vx[i];
+  if (q == 1 && nb <= 1) {
+    double f = 0.0;
+    if (!factor0) f = wet_dry_factor(P, hk, hlo, dmax(dmax(h0, dmax(h1, h2)), hk));
+    s_factor[lane] = f;
+    if (ORD && in) d.cls[k] = (unsigned char)((dry ? 1 : 0) | (dbits(f) == dbits(1.0) ? 0 : 2));
+  } else if (q == 1 && ORD && in) {
+    d.cls[k] = (unsigned char)(dry ? 1 : 0);
   }
+  if (grad) edge_jumps(qc, q0, q1, q2, G, jump, lo, hi);
+  __syncthreads();
+  E[0] = E[1] = E[2] = qc;
+  if (grad) {
+    const double f = s_factor[lane];
+    // at factor 1 the betas and their reciprocals are the precomputed ones
+    const bool one = dbits(f) == dbits(1.0);
+    const double beta1 = q < 2 ? P.beta_w1 : q == 2 ? P.beta_uh1 : P.beta_vh1;
+    const double inv1 = q < 2 ? P.inv_beta_w1 : q == 2 ? P.inv_beta_uh1 : P.inv_beta_vh1;
+    const double beta = one ? beta1 : beta0_dry + (beta0 - beta0_dry) * f;
+    if (dgt0(beta)) limited_edges(qc, jump, limiter_phi(jump, lo, hi, beta, one ? inv1 : 0.0), E);
+  } else if (nb == 2) {
+    const double qn = s.x != k ? q0 : (s.y != k ? q1 : q2);
+    reconstruct_towards(P.beta_w, P.inv_beta_w, qc, qn, G, E);
+  }
+  if (q == 1) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) s_h[i][lane] = E[i];
+  }
+  __syncthreads();
+  if (!in) return;
+  const size_t b = 3 * (size_t)k;
+  if (q >= 2 && P.velocity_extrapolation) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) E[i] = E[i] * s_h[i][lane];
+  }
+  double* const out = q == 0 ? d.we : q == 1 ? d.he : q == 2 ? d.uhe : d.vhe;
+#pragma unroll
+  for (int i = 0; i < 3; i++) out[b + i] = E[i];
+  if (q >= 2 && sdry) (q == 2 ? d.uh : d.vh)[k] = 0.0;
+  double vx[3];
   if (VERT) {
-    double vx[3];
-    vertex_from_edges(E.w, vx);
-    for (int i = 0; i < 3; i++) d.wv[b + i] = vx[i];
-    vertex_from_edges(E.h, vx);
-    for (int i = 0; i < 3; i++) d.hv[b + i] = vx[i];
-    vertex_from_edges(E.uh, vx);
-    for (int i = 0; i < 3; i++) d.uhv[b + i] = vx[i];
-    vertex_from_edges(E.vh, vx);
-    for (int i = 0; i < 3; i++) d.vhv[b + i] = vx[i];
-    vertex_from_edges(E.z, vx);
-    for (int i = 0; i < 3; i++) d.zv[b + i] = vx[i];
+    double* const vert = q == 0 ? d.wv : q == 1 ? d.hv : q == 2 ? d.uhv : d.vhv;
+    vertex_from_edges(E, vx);
+    for (int i = 0; i < 3; i++) vert[b + i] = vx[i];
   }
+  if (q == 0) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      E[i] = E[i] - s_h[i][lane];
+      d.ze[b + i] = E[i];
+    }
+    if (VERT || P.sloped_mannings) {       // sloped friction reads the bed vertex values
+      vertex_from_edges(E, vx);
+      for (int i = 0; i < 3; i++) d.zv[b + i] = vx[i];
+    }
+  }
+}
+
+// The extrapolation geometry from the caller's rows [N][GEO_STRIDE] to one
+// array per coefficient, so that the lanes of a warp read it contiguously.
+__global__ void k_geo_transpose(double* out, const double* rows, int N) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= N) return;
+#pragma unroll
+  for (int i = 0; i < GEO_STRIDE; i++) out[(size_t)i * N + k] = rows[(size_t)GEO_STRIDE * k + i];
 }
 
 __global__ void k_order_init(Dev d) {
@@ -633,6 +687,7 @@ __global__ void k_store_bfs(Dev d, int substep) {
 
 // ---------------------------------------------------------------------------
 static inline int nblk(int n) { return (n + TPB - 1) / TPB; }
+static inline int xblk(int n) { return (n + XCELLS - 1) / XCELLS; }
 
 #define LAUNCHK(cat, ...)                  \
   do {                                     \
@@ -653,8 +708,8 @@ cudaError_t enqueue_distribute(Scenario* s, cudaStream_t st, bool with_protect, 
   const Dev& d = s->d;
   if (d.N == 0) return cudaSuccess;
   LAUNCHK(PH_PREP, k_prep<<<nblk(d.N), TPB, 0, st>>>(d, with_protect ? 0 : 2));
-  if (vertices) LAUNCHK(PH_EXTRAP, k_extrap<true><<<nblk(d.N), TPB, 0, st>>>(d));
-  else LAUNCHK(PH_EXTRAP, k_extrap<false><<<nblk(d.N), TPB, 0, st>>>(d));
+  if (vertices) LAUNCHK(PH_EXTRAP, k_extrap<true><<<xblk(d.N), XTPB, 0, st>>>(d));
+  else LAUNCHK(PH_EXTRAP, k_extrap<false><<<xblk(d.N), XTPB, 0, st>>>(d));
   return cudaSuccess;
 }
 
@@ -715,26 +770,27 @@ cudaError_t enqueue_saxpy(Scenario* s, cudaStream_t st, double a, double b) {
 }
 
 // One full timestep (Euler, RK2 or RK3), ending with the clock kernel.
+cudaError_t enqueue_geo_transpose(Scenario* s, cudaStream_t st, const double* rows) {
+  if (s->d.N == 0) return cudaSuccess;
+  LAUNCH(k_geo_transpose<<<nblk(s->d.N), TPB, 0, st>>>((double*)s->d.geo, rows, s->d.N));
+  return cudaSuccess;
+}
+
 cudaError_t enqueue_order_init(Scenario* s, cudaStream_t st) {
   if (s->d.N == 0) return cudaSuccess;
   LAUNCH(k_order_init<<<nblk(s->d.N), TPB, 0, st>>>(s->d));
   return cudaSuccess;
 }
 
-// The step's extrapolation; with AGX_EXTRAP_ORDER it visits the cells in the
-// order of the previous one's classes and sorts them by this one's.
+// The step's extrapolation: visits the cells in the order of the branch
+// classes the previous step recorded; the step's last one sorts them again.
 static cudaError_t enqueue_step_extrap(const Dev& d, cudaStream_t st, bool last) {
-  const int nb = nblk(d.N);
-  if (AGX_EXTRAP_ORDER) {
+  LAUNCHK(PH_EXTRAP, k_extrap<false, true><<<xblk(d.N), XTPB, 0, st>>>(d));
+  if (last) {
     const int sb = (d.N + SORT_SPAN - 1) / SORT_SPAN;
-    LAUNCHK(PH_EXTRAP, k_extrap<false, true><<<nb, TPB, 0, st>>>(d));
-    if (last || AGX_SORT_CADENCE == 1) {
-      LAUNCH(k_cls_count<<<sb, TPB, 0, st>>>(d));
-      LAUNCH(k_cls_offsets<<<1, 256, 0, st>>>(d));
-      LAUNCH(k_cls_scatter<<<sb, TPB, 0, st>>>(d));
-    }
-  } else {
-    LAUNCHK(PH_EXTRAP, k_extrap<false><<<nb, TPB, 0, st>>>(d));
+    LAUNCH(k_cls_count<<<sb, TPB, 0, st>>>(d));
+    LAUNCH(k_cls_offsets<<<1, 256, 0, st>>>(d));
+    LAUNCH(k_cls_scatter<<<sb, TPB, 0, st>>>(d));
   }
   return cudaSuccess;
 }

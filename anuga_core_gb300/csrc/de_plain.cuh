@@ -303,13 +303,10 @@ AGX_HD void limited_edges(double qc, const double jump[3], double phi, double ou
   }
 }
 
-// Returns the limiter's phi (1 where the reconstruction is not limited).
-AGX_HD double reconstruct3(double beta, double inv_known, double qc, double q0, double q1, double q2,
-                           const double* G, double out[3]) {
-  if (!dgt0(beta)) {
-    out[0] = qc; out[1] = qc; out[2] = qc;
-    return 1.0;
-  }
+// The jumps to the three edges (the auxiliary triangle's gradient over the
+// edge offsets) and the admissible jump range [lo, hi].
+AGX_HD void edge_jumps(double qc, double q0, double q1, double q2, const double G[GEO_STRIDE], double jump[3],
+                       double& lo, double& hi) {
   const double d0 = q0 - qc;
   const double d1 = q1 - q0;
   const double d2 = q2 - q0;
@@ -317,16 +314,12 @@ AGX_HD double reconstruct3(double beta, double inv_known, double qc, double q0, 
   gx *= G[10];
   double gy = G[6] * d2 - G[7] * d1;
   gy *= G[10];
-  double jump[3];
   for (int i = 0; i < 3; i++) jump[i] = gx * G[i] + gy * G[3 + i];
-  const double hi = dmax(dmax(d0, dmax(d0 + d1, d0 + d2)), 0.0);
-  const double lo = dmin(dmin(d0, dmin(d0 + d1, d0 + d2)), 0.0);
-  const double phi = limiter_phi(jump, lo, hi, beta, inv_known);
-  limited_edges(qc, jump, phi, out);
-  return phi;
+  hi = dmax(dmax(d0, dmax(d0 + d1, d0 + d2)), 0.0);
+  lo = dmin(dmin(d0, dmin(d0 + d1, d0 + d2)), 0.0);
 }
 
-AGX_HD void reconstruct_towards(double beta, double inv_known, double qc, double qn, const double* G,
+AGX_HD void reconstruct_towards(double beta, double inv_known, double qc, double qn, const double G[GEO_STRIDE],
                                 double out[3]) {
   const double d = qn - qc;
   const double gx = d * G[6];
@@ -339,9 +332,31 @@ AGX_HD void reconstruct_towards(double beta, double inv_known, double qc, double
   limited_edges(qc, jump, phi, out);
 }
 
+// A non-negative double cut to the float below it; 0 below the float range.
+AGX_HD float cut_to_float(double x) {
+  const int64_t b = dbits(x);
+  const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
+  const uint32_t f = hi < 0x38100000u ? 0u : ((hi - 0x38000000u) << 3) | (lo >> 29);
+  float r;
+#ifdef __CUDA_ARCH__
+  r = __uint_as_float(f);
+#else
+  memcpy(&r, &f, sizeof r);
+#endif
+  return r;
+}
+
 // Wet/dry blending factor (:1537-1551).  In deep water it is exactly 1 and
-// is decided by comparisons with margin instead of the three divisions.
+// is decided by comparisons with margin instead of the three divisions:
+// first in FP32 with a margin of 3e-4, far above the cut's 2^-23, then (where
+// that does not settle it) in FP64 with a margin of 2^-40.
 AGX_HD double wet_dry_factor(const Params& P, double hc, double hlo, double hhi) {
+  if (dbits(hlo) >= 0 && dkey(hhi) < (int64_t)0x4700000000000000ll) {       // 0 <= hlo <= hc <= hhi < 2^113
+    const float fc = cut_to_float(hc), flo = cut_to_float(hlo), fhi = cut_to_float(hhi);
+    if (flo >= 0.3001f * fmaxf(fc, 1.0e-06f) && fc >= 0.3001f * fmaxf(fhi, 1.0e-06f) && flo >= 1.0e-30f &&
+        flo >= 11.01f * cut_to_float(P.hmin))
+      return 1.0;
+  }
   const double m = 1.0 + 9.094947017729282e-13;
   const double hc_e = dmax(hc, 1.0e-06);
   const double hhi_e = dmax(hhi, 1.0e-06);
@@ -367,10 +382,6 @@ AGX_HD bool surrounded_dry(const Params& P, int s, const int4* surr, const doubl
          (dlt(h[q.z], P.hmin) | (q.z == s));
 }
 
-struct EdgeOut {       // edge values of one cell, slots 0..2
-  double w[3], h[3], uh[3], vh[3], z[3];
-};
-
 // Reconstruction value of neighbour s as seen from cell k: the reference's
 // in-order loop has already zeroed the velocity of a surrounded-dry cell s
 // that precedes k.  Only consulted where that value can matter.
@@ -382,87 +393,6 @@ AGX_HD void neighbour_uv(const Params& P, int s, bool before, const int4* surr, 
     us = 0.0;
     vs = 0.0;
   }
-}
-
-// Main extrapolation loop body (:1418-1896) for cell k.  Returns true if the
-// cell's centroid momenta must be zeroed (surrounded by dry cells).  *cls
-// (if given) receives the branches the cell took: bits 0-1 the boundary
-// class (0: at most one boundary edge, 1: two, 2: three), bit 2 a dry cell,
-// bit 3 a wet/dry factor below 1, bits 4-7 a limited stage, height,
-// x and y reconstruction.
-AGX_HD bool extrap_cell(const Params& P, int k, const int4* conn, const int4* surr, const double* geo,
-                        const double* w, const double* h, const double* u, const double* v,
-                        EdgeOut& E, int* cls = nullptr) {
-  const int4 s = surr[k];
-  const int meta = conn[k].w;
-  const int nb = meta_nb(meta);
-  const double* G = geo + (size_t)GEO_STRIDE * k;
-  const double hk = h[k];
-  const bool sdry = (dlt(h[s.x], P.hmin) | (s.x == k)) & (dlt(h[s.y], P.hmin) | (s.y == k)) &
-                    (dlt(h[s.z], P.hmin) | (s.z == k));
-  double uk = u[k], vk = v[k];
-  if (sdry) { uk = 0.0; vk = 0.0; }
-  int c = (nb == 3 ? 2 : (nb == 2 ? 1 : 0)) | (dlt(hk, P.hmin) ? 4 : 0);
-  if (nb == 3) {
-    for (int i = 0; i < 3; i++) {
-      E.w[i] = w[k]; E.uh[i] = uk; E.vh[i] = vk; E.h[i] = hk;
-    }
-  } else if (nb <= 1) {
-    const double h0 = h[s.x], h1 = h[s.y], h2 = h[s.z];
-    const double hlo = dmin(dmin(h0, dmin(h1, h2)), hk);
-    const double hhi = dmax(dmax(h0, dmax(h1, h2)), hk);
-    const double hf = wet_dry_factor(P, hk, hlo, hhi);
-    // at hf == 1 the betas and their reciprocals are the precomputed ones
-    const bool one = dbits(hf) == dbits(1.0);
-    const double beta = one ? P.beta_w1 : P.beta_w_dry + (P.beta_w - P.beta_w_dry) * hf;
-    const double ib = one ? P.inv_beta_w1 : 0.0;
-    const double pw = reconstruct3(beta, ib, w[k], w[s.x], w[s.y], w[s.z], G, E.w);
-    const double ph = reconstruct3(beta, ib, hk, h0, h1, h2, G, E.h);
-    const double beta_u = one ? P.beta_uh1 : P.beta_uh_dry + (P.beta_uh - P.beta_uh_dry) * hf;
-    const double beta_v = one ? P.beta_vh1 : P.beta_vh_dry + (P.beta_vh - P.beta_vh_dry) * hf;
-    double u0 = u[s.x], u1 = u[s.y], u2 = u[s.z];
-    double v0 = v[s.x], v1 = v[s.y], v2 = v[s.z];
-    // Neighbour velocities can be stale-zeroed only for a dry cell k (a wet
-    // neighbour rules out "surrounded by dry"); they matter only if the dry
-    // reconstruction has a positive beta.
-    if (dlt(hk, P.hmin) && (dgt0(beta_u) || dgt0(beta_v))) {
-      neighbour_uv(P, s.x, meta_before(meta, 0) && s.x != k, surr, h, u, v, u0, v0);
-      neighbour_uv(P, s.y, meta_before(meta, 1) && s.y != k, surr, h, u, v, u1, v1);
-      neighbour_uv(P, s.z, meta_before(meta, 2) && s.z != k, surr, h, u, v, u2, v2);
-      if (s.x == k) { u0 = uk; v0 = vk; }
-      if (s.y == k) { u1 = uk; v1 = vk; }
-      if (s.z == k) { u2 = uk; v2 = vk; }
-    } else {
-      if (s.x == k) { u0 = uk; v0 = vk; }
-      if (s.y == k) { u1 = uk; v1 = vk; }
-      if (s.z == k) { u2 = uk; v2 = vk; }
-    }
-    const double pu = reconstruct3(beta_u, one ? P.inv_beta_uh1 : 0.0, uk, u0, u1, u2, G, E.uh);
-    const double pv = reconstruct3(beta_v, one ? P.inv_beta_vh1 : 0.0, vk, v0, v1, v2, G, E.vh);
-    c |= (one ? 0 : 8) | (dbits(pw) != dbits(1.0) ? 16 : 0) | (dbits(ph) != dbits(1.0) ? 32 : 0) |
-         (dbits(pu) != dbits(1.0) ? 64 : 0) | (dbits(pv) != dbits(1.0) ? 128 : 0);
-  } else {
-    int j = 0;
-    const int sv[3] = {s.x, s.y, s.z};
-    while (j < 2 && sv[j] == k) j++;
-    const int kn = sv[j];
-    reconstruct_towards(P.beta_w, P.inv_beta_w, w[k], w[kn], G, E.w);
-    reconstruct_towards(P.beta_w, P.inv_beta_w, hk, h[kn], G, E.h);
-    double un, vn;
-    neighbour_uv(P, kn, meta_before(meta, j) != 0, surr, h, u, v, un, vn);
-    reconstruct_towards(P.beta_w, P.inv_beta_w, uk, un, G, E.uh);
-    reconstruct_towards(P.beta_w, P.inv_beta_w, vk, vn, G, E.vh);
-  }
-  if (P.velocity_extrapolation) {
-    for (int i = 0; i < 3; i++) {
-      const double dk = E.h[i];
-      E.uh[i] = E.uh[i] * dk;
-      E.vh[i] = E.vh[i] * dk;
-    }
-  }
-  for (int i = 0; i < 3; i++) E.z[i] = E.w[i] - E.h[i];
-  if (cls) *cls = c;
-  return sdry;
 }
 
 AGX_HD void vertex_from_edges(const double e[3], double vx[3]) {
