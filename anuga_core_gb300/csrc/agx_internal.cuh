@@ -27,7 +27,8 @@ struct Clock {
   long long steps_call, total_steps, steps_target, negative_cells;
   long long nonfinite_cells;             // cell updates that produced a NaN or an infinity
   int smallsteps, max_smallsteps, order, default_order;
-  int error, reason, fluxcalls, pad1;    // fluxcalls: stages per step (1 euler, 2 rk2, 3 rk3)
+  int error, reason, fluxcalls;          // fluxcalls: stages per step (1 euler, 2 rk2, 3 rk3)
+  unsigned blocks_done;                  // blocks of the running kernel that have finished (0 between kernels)
   double bf_integral;                    // time integral of the boundary flux sums
   double fixed_flux_dt;                  // > 0: set_fixed_flux_timestep (replaces the CFL minimum)
   double op_influx[MAX_OPS];
@@ -182,12 +183,6 @@ struct Dev {
   double *sw, *suh, *svh;
   double *max_speed;
   double *sl0, *sl1, *sl2, *slsp, *slpf, *slhl;
-  // the extrapolation's cell order: cells grouped by the branches they took
-  // in the previous extrapolation (cls), so that the lanes of a warp follow
-  // the same path; cls_count[0..255] counts, [256..511] scatter cursors
-  int* order;
-  unsigned char* cls;
-  unsigned int* cls_count;
   Clock* clock;
   // riverwalls (structures/riverwall.py): per slot the 1-based riverwall
   // edge (0: ordinary edge), crest elevation and hydraulic-table row per
@@ -262,15 +257,13 @@ cudaError_t enqueue_rate_once(Scenario* s, cudaStream_t st, int op, double rate,
 cudaError_t enqueue_op(Scenario* s, cudaStream_t st, int op, double rate, double factor, double dt);
 cudaError_t enqueue_sww_frame(Scenario* s, cudaStream_t st, double min_storable_height, int centroid_avg);
 cudaError_t enqueue_protect(Scenario* s, cudaStream_t st);
-cudaError_t enqueue_boundary(Scenario* s, cudaStream_t st, double t_override, bool stage2);
+cudaError_t enqueue_boundary(Scenario* s, cudaStream_t st, double t_override);
 cudaError_t enqueue_fluxes(Scenario* s, cudaStream_t st, int substep);
 cudaError_t enqueue_update(Scenario* s, cudaStream_t st, int stage, bool use_clock_dt, double dt);
 cudaError_t enqueue_forcing(Scenario* s, cudaStream_t st);
 cudaError_t enqueue_backup(Scenario* s, cudaStream_t st);
 cudaError_t enqueue_saxpy(Scenario* s, cudaStream_t st, double a, double b);
 cudaError_t enqueue_divide(Scenario* s, cudaStream_t st, double divisor);
-cudaError_t enqueue_reset_accum(Scenario* s, cudaStream_t st);
-cudaError_t enqueue_order_init(Scenario* s, cudaStream_t st);
 cudaError_t enqueue_geo_transpose(Scenario* s, cudaStream_t st, const double* rows);
 
 }  // namespace agx

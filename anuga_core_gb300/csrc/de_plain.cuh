@@ -167,32 +167,26 @@ AGX_HD void finish_params(Params& P) {
 // extrapolation (:1373-1402).  Writes the protected stage, zeroes momenta of
 // (near-)dry cells, and the depth and reconstruction variable (velocity or
 // momentum).  Returns the mass added by protection.
-AGX_HD double prep_cell(const Params& P, int k, double* w, double* uh, double* vh,
-                        const double* z, const double* area, double* h, double* u, double* v,
-                        bool do_protect = true, bool do_prep = true) {
-  double wk = w[k];
-  const double zk = z[k];
-  double uk = uh[k], vk = vh[k];
+// On values: wk, uk, vk in and out, area read only where mass is added.
+AGX_HD double prep_values(const Params& P, double& wk, double& uk, double& vk, double zk, const double* area,
+                          double& dk, double& ru, double& rv, bool do_protect = true, bool do_prep = true) {
   double added = 0.0;
-  const double depth = wk - zk;
+  double depth = wk - zk;
   if (do_protect && dlt(depth, P.hmin * 1.0)) {
     uk = 0.0;
     if (P.protect_zero_ymom) vk = 0.0;
     if (dle0(depth)) {
       if (dlt(wk, zk)) {
-        added = (zk - wk) * area[k];
+        added = (zk - wk) * *area;
         wk = zk;
+        depth = 0.0;             // zk - zk (a depth of -0 elsewhere becomes +0 below)
       }
     }
   }
-  if (!do_prep) {
-    w[k] = wk;
-    uh[k] = uk;
-    vh[k] = vk;
-    return added;
-  }
-  const double dk = dmax(wk - zk, 0.0);
-  double ru = 0.0, rv = 0.0;
+  if (!do_prep) return added;
+  dk = dmax(depth, 0.0);
+  ru = 0.0;
+  rv = 0.0;
   if (dle(dk, P.hmin)) {
     uk = 0.0;
     vk = 0.0;
@@ -204,12 +198,22 @@ AGX_HD double prep_cell(const Params& P, int k, double* w, double* uh, double* v
     ru = uk;
     rv = vk;
   }
+  return added;
+}
+
+AGX_HD double prep_cell(const Params& P, int k, double* w, double* uh, double* vh,
+                        const double* z, const double* area, double* h, double* u, double* v,
+                        bool do_protect = true, bool do_prep = true) {
+  double wk = w[k], uk = uh[k], vk = vh[k], dk, ru, rv;
+  const double added = prep_values(P, wk, uk, vk, z[k], area + k, dk, ru, rv, do_protect, do_prep);
   w[k] = wk;
   uh[k] = uk;
   vh[k] = vk;
-  h[k] = dk;
-  u[k] = ru;
-  v[k] = rv;
+  if (do_prep) {
+    h[k] = dk;
+    u[k] = ru;
+    v[k] = rv;
+  }
   return added;
 }
 
