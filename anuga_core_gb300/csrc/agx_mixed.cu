@@ -592,8 +592,9 @@ __device__ __forceinline__ void flux_phase(const PoolDev& d, EdgeState* es) {
         const EdgeState L = es[threadIdx.x * 3 + i];   // own edge from the staging (fewer live registers)
         const int n = nbr[i];
         float hre, uhr, vhr, dd = 0.0f;
-        const float len = sqrtf(evx[i] * evx[i] + evy[i] * evy[i]);
-        const float il = 1.0f / len;
+        const float l2 = evx[i] * evx[i] + evy[i] * evy[i];
+        const float len = sqrtf(l2);
+        const float il = rsqrtf(l2);
         const float n1 = evy[i] * il, n2 = -evx[i] * il;
         if (n >= 0) {
           const int m = nedge_of(cn.w, i);

@@ -39,15 +39,19 @@ struct EdgeState {          // one edge of one cell, relative to that cell
   float dz;                 // bed at the edge minus the cell's centroid bed
 };
 
+// __limit_gradient's phi: the smallest of hi / J over the jumps above +tiny
+// and lo / J over those below -tiny (1 with the first jump between them,
+// else 1000, where there is none), times beta, at most 1.  hi and lo are the
+// same for every slot, so the largest and the smallest jump give the minimum
+// and two quotients stand for up to six.
 __device__ __forceinline__ float limiter_phi32(const float J[3], float lo, float hi, float beta) {
   const float tiny = 1.0e-30f;
-  float r = 1000.0f, cand = 1.0f;
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    if (J[i] < -tiny) cand = lo / J[i];
-    if (J[i] > tiny) cand = hi / J[i];
-    r = fminf(cand, r);
-  }
+  const float up = fmaxf(fmaxf(J[0], J[1]), J[2]);
+  const float down = fminf(fminf(J[0], J[1]), J[2]);
+  float r = fabsf(J[0]) <= tiny ? 1.0f : 1000.0f;
+  const float qu = __fdividef(hi, up), qd = __fdividef(lo, down);
+  r = up > tiny ? fminf(qu, r) : r;
+  r = down < -tiny ? fminf(qd, r) : r;
   return fminf(r * beta, 1.0f);
 }
 
@@ -68,9 +72,9 @@ __device__ __forceinline__ void limited_jumps(const float M[9], const float D[3]
 }
 
 __device__ __forceinline__ float wet_dry_factor32(const MParams& P, float hc, float hlo, float hhi) {
-  float f = fmaxf(0.0f, fminf(P.c_tmp * fmaxf(hlo, 0.0f) / fmaxf(hc, 1.0e-06f) + P.d_tmp,
-                              fminf(P.c_tmp * fmaxf(hc, 0.0f) / fmaxf(hhi, 1.0e-06f) + P.d_tmp, 1.0f)));
-  f = fminf(1.2f * fmaxf(hlo - P.hmin, 0.0f) / (fmaxf(hlo, 0.0f) + 1.0f * P.hmin), f);
+  float f = fmaxf(0.0f, fminf(__fdividef(P.c_tmp * fmaxf(hlo, 0.0f), fmaxf(hc, 1.0e-06f)) + P.d_tmp,
+                              fminf(__fdividef(P.c_tmp * fmaxf(hc, 0.0f), fmaxf(hhi, 1.0e-06f)) + P.d_tmp, 1.0f)));
+  f = fminf(__fdividef(1.2f * fmaxf(hlo - P.hmin, 0.0f), fmaxf(hlo, 0.0f) + P.hmin), f);
   return f;
 }
 
