@@ -569,7 +569,9 @@ __device__ __forceinline__ void flux_phase(const PoolDev& d, EdgeState* es) {
     // every term the loop below would add is +0 (both Audusse depths are
     // zero, so the flux, the speed and the pressure terms vanish), so the
     // loop and its geometry loads are skipped with the same result.
-    bool dry = valid && cn.x >= 0 && cn.y >= 0 && cn.z >= 0 && !(EXT && ((cn.w >> 20) & 7));
+    // Looked at only where the cell itself is dry: a wet cell's edge depths
+    // are all zero by accident at most, and the loop gives the same.
+    bool dry = valid && rk.x == 0.0f && cn.x >= 0 && cn.y >= 0 && cn.z >= 0 && !(EXT && ((cn.w >> 20) & 7));
     if (dry) {
 #pragma unroll
       for (int i = 0; i < 3; i++) {
