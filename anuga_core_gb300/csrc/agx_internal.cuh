@@ -141,6 +141,19 @@ __host__ __device__ inline int clock_logic(Clock* c) {
   return reason;
 }
 
+// The last block of a kernel to finish runs timestep_logic or clock_logic
+// itself.  Its SM's L1 may hold lines of the clock from before the other
+// blocks' atomics, so the fields these change are read past it and stored
+// back, which the thread's own later loads see; no other field changes while
+// the kernel runs.
+__device__ __forceinline__ void clock_refresh(Clock* c) {
+  c->error = __ldcg(&c->error);
+  c->bfs_acc = __ldcg(&c->bfs_acc);
+  c->bfs[1] = __ldcg(&c->bfs[1]);
+  c->bfs[2] = __ldcg(&c->bfs[2]);
+  c->dt_key = __ldcg(&c->dt_key);
+}
+
 // A fractional-step operator: Rate_operator (kind 0) or Inlet_operator
 // (kind 1: rate = constant discharge Q, vu/vv the imposed velocity when
 // flags & 1, zero velocity when flags & 2, area = the inlet's total area).

@@ -93,36 +93,22 @@ __device__ __forceinline__ bool last_to_finish(Clock* c) {
   return atomicAdd(&c->blocks_done, 1u) == gridDim.x - 1;
 }
 
-// The clock as the other blocks left it: read past this SM's L1, which may
-// hold lines of it from before their atomics.
-__device__ __forceinline__ void clock_read(Clock& c, const Clock* g) {
-  static_assert(sizeof(Clock) % 8 == 0, "the clock is read in 8-byte words");
-  const unsigned long long* s = reinterpret_cast<const unsigned long long*>(g);
-  unsigned long long* t = reinterpret_cast<unsigned long long*>(&c);
-#pragma unroll 8
-  for (int i = 0; i < (int)(sizeof(Clock) / 8); i++) t[i] = __ldcg(s + i);
-}
-
 // After the accumulation: the stage's boundary flux sum, and at a step's
 // first stage its timestep.
-__device__ __noinline__ void finish_accum(Clock* g, int substep, int timestep) {
+__device__ __noinline__ void finish_accum(Clock* c, int substep, int timestep) {
   __threadfence();
-  Clock c;
-  clock_read(c, g);
-  c.bfs[substep] = c.bfs_acc;
-  if (timestep) timestep_logic(&c);
-  c.blocks_done = 0u;
-  *g = c;
+  clock_refresh(c);
+  c->bfs[substep] = c->bfs_acc;
+  if (timestep) timestep_logic(c);
+  c->blocks_done = 0u;
 }
 
 // After the step's last update: the clock and the graph's while condition.
-__device__ __noinline__ void finish_step(Clock* g, cudaGraphConditionalHandle handle, int set_cond) {
+__device__ __noinline__ void finish_step(Clock* c, cudaGraphConditionalHandle handle, int set_cond) {
   __threadfence();
-  Clock c;
-  clock_read(c, g);
-  const int reason = clock_logic(&c);
-  c.blocks_done = 0u;
-  *g = c;
+  clock_refresh(c);
+  const int reason = clock_logic(c);
+  c->blocks_done = 0u;
   if (set_cond) cudaGraphSetConditional(handle, reason == 0 ? 1u : 0u);
 }
 
