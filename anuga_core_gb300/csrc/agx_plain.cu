@@ -340,17 +340,23 @@ __global__ void __launch_bounds__(TPB, AGX_MINB_FLUX) k_flux(const __grid_consta
   double hr;
   slot_flux(d.P, k, i, cn, d.we, d.uhe, d.vhe, d.ze, d.he, d.wb, d.uhb, d.vhb, d.normals, d.w,
             d.h, d.z, RW, R, hr);
-  d.sl0[s] = R.f[0];
-  d.sl1[s] = R.f[1];
-  d.sl2[s] = R.f[2];
+  // the contributions -f * length of the edge's two cells (opposite but for
+  // the length, which a table could hold differently for the two sides)
+  const double len = d.lengths[s];
+  const double e0 = dneg(R.f[0]) * len, e1 = dneg(R.f[1]) * len, e2 = dneg(R.f[2]) * len;
+  d.sl0[s] = e0;
+  d.sl1[s] = e1;
+  d.sl2[s] = e2;
   d.slsp[s] = R.speed;
   d.slpf[s] = R.pflux;
   d.slhl[s] = R.hleft;
   const int o = d.edge_opp[e];
   if (o >= 0) {
-    d.sl0[o] = -R.f[0];
-    d.sl1[o] = -R.f[1];
-    d.sl2[o] = -R.f[2];
+    const double len_o = d.lengths[o];
+    const bool same = dbits(len_o) == dbits(len);
+    d.sl0[o] = same ? dneg(e0) : R.f[0] * len_o;
+    d.sl1[o] = same ? dneg(e1) : R.f[1] * len_o;
+    d.sl2[o] = same ? dneg(e2) : R.f[2] * len_o;
     d.slsp[o] = R.speed;
     d.slpf[o] = R.pflux;
     d.slhl[o] = hr;
@@ -394,7 +400,7 @@ __global__ void __launch_bounds__(TPB, AGX_MINB_ACCUM) k_accum(Dev d, int subste
       F.smax = 0.0;
       F.bflux = 0.0;
     } else {
-      accum_cell(d.P, k, c, R, d.he, d.ze, d.h, d.z, d.normals, d.lengths, d.inv_area[k], fn, F);
+      accum_cell<true>(d.P, k, c, R, d.he, d.ze, d.h, d.z, d.normals, d.lengths, d.inv_area[k], fn, F);
     }
     d.xw[k] = F.ew;
     d.xuh[k] = F.euh;
@@ -439,8 +445,8 @@ __global__ void __launch_bounds__(TPB, AGX_MINB_UPDATE) k_update(Dev d, int stag
       double S;
       if (d.P.sloped_mannings) S = manning_S_sloped(d.P, w, d.zv + 3 * (size_t)k, d.vcoord + 6 * (size_t)k, uh, vh, d.eta[k]);
       else S = manning_S(d.P, w, z, uh, vh, d.eta[k]);
-      suh += S * uh;
-      svh += S * vh;
+      suh = dnz(suh) ? suh + S * uh : S * uh;     // 0 + x: a zero's sign plays no part in the update
+      svh = dnz(svh) ? svh + S * vh : S * vh;
     }
     if (!update_quantity(w, d.xw[k], sw, dt)) bad = 1;
     if (!update_quantity(uh, d.xuh[k], suh, dt)) bad = 1;
@@ -451,9 +457,13 @@ __global__ void __launch_bounds__(TPB, AGX_MINB_UPDATE) k_update(Dev d, int stag
       uh = 0.0;
       vh = 0.0;
     }
-    if (saxpy) {
-      const double a = saxpy == 2 ? 0.25 : (saxpy == 3 ? 2.0 : 0.5);
-      const double b = saxpy == 2 ? 0.75 : (saxpy == 3 ? 1.0 : 0.5);
+    if (saxpy == 1) {
+      w = dhalf_sum(w, d.w0[k]);
+      uh = dhalf_sum(uh, d.uh0[k]);
+      vh = dhalf_sum(vh, d.vh0[k]);
+    } else if (saxpy) {
+      const double a = saxpy == 2 ? 0.25 : 2.0;
+      const double b = saxpy == 2 ? 0.75 : 1.0;
       w = a * w + b * d.w0[k];
       uh = a * uh + b * d.uh0[k];
       vh = a * vh + b * d.vh0[k];

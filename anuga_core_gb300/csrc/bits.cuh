@@ -11,7 +11,7 @@
 
 #ifdef __CUDACC__
 #define AGX_BITS __host__ __device__ __forceinline__
-#define AGX_BITS_COLD __host__ __device__ __noinline__
+#define AGX_BITS_COLD static __host__ __device__ __noinline__
 #else
 #define AGX_BITS inline
 #define AGX_BITS_COLD __attribute__((noinline))

@@ -41,6 +41,7 @@
 #include <string.h>
 #include <math.h>
 #include "soft64.cuh"
+#include "bits.cuh"
 
 #ifdef __CUDACC__
 #define AGX_HD __host__ __device__ __forceinline__
@@ -79,6 +80,17 @@ AGX_HD bool dle0(double x) { return dkey(x) <= 0; }             // x <= 0
 AGX_HD bool dnz(double x) { return ((uint64_t)dbits(x) << 1) != 0; }   // x != 0
 AGX_HD double dmax(double a, double b) { return dkey(a) >= dkey(b) ? a : b; }
 AGX_HD double dmin(double a, double b) { return dkey(a) <= dkey(b) ? a : b; }
+
+// -x by its sign bit (a negation stored as it is takes the FP64 pipe).
+AGX_HD double dneg(double x) {
+#ifdef __CUDA_ARCH__
+  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
+#else
+  return -x;
+#endif
+}
+// 0.0 + x: x itself, but +0 for -0 (the first term of a sum).
+AGX_HD double dplus0(double x) { return dnz(x) ? x : 0.0; }
 
 // ---- FP64 division and square root ----------------------------------------
 // Correctly rounded either way, so the results are the same bits.
@@ -147,6 +159,7 @@ struct Params {
   // positive, divided out per cell)
   double beta_w1, beta_uh1, beta_vh1;
   double inv_beta_w1, inv_beta_uh1, inv_beta_vh1, inv_beta_w;
+  double half_g;                // 0.5 * g (exact)
 };
 
 AGX_HD double positive_inverse(double b) { return b > 0.0 ? 1.0 / b : 0.0; }
@@ -160,6 +173,7 @@ AGX_HD void finish_params(Params& P) {
   P.inv_beta_uh1 = positive_inverse(P.beta_uh1);
   P.inv_beta_vh1 = positive_inverse(P.beta_vh1);
   P.inv_beta_w = positive_inverse(P.beta_w);
+  P.half_g = 0.5 * P.g;
 }
 
 // ---- protect + depth/velocity preparation --------------------------------
@@ -414,7 +428,7 @@ struct FluxOut {
 
 AGX_HD void central_flux(const double ql[3], const double qr[3], double hl, double hr,
                          double hle, double hre, double n1, double n2, double eps, double ze,
-                         double g, int low_froude, FluxOut& F) {
+                         double g, double half_g, int low_froude, FluxOut& F) {
   if (!dnz(hl) && !dnz(hr)) {
     F.f[0] = F.f[1] = F.f[2] = 0.0;
     F.speed = 0.0;
@@ -426,24 +440,24 @@ AGX_HD void central_flux(const double ql[3], const double qr[3], double hl, doub
   double vhl = -n2 * ql[1] + n1 * ql[2];
   double uhr = n1 * qr[1] + n2 * qr[2];
   double vhr = -n2 * qr[1] + n1 * qr[2];
-  double ul, vl, ur, vr;
+  double ul, vl = 0.0, ur, vr = 0.0;         // vl, vr: read by the low-Froude scaling only
   if (dgt0(hle)) {
     const double inv = ddiv(1.0, hle);
     ul = uhl * inv;
     uhl = hl * ul;
-    vl = vhl * inv;
+    if (low_froude) vl = vhl * inv;
     vhl = hl * inv * vhl;
   } else {
-    ul = uhl = vhl = vl = 0.0;
+    ul = uhl = vhl = 0.0;
   }
   if (dgt0(hre)) {
     const double inv = ddiv(1.0, hre);
     ur = uhr * inv;
     uhr = hr * ur;
-    vr = vhr * inv;
+    if (low_froude) vr = vhr * inv;
     vhr = hr * inv * vhr;
   } else {
-    ur = uhr = vhr = vr = 0.0;
+    ur = uhr = vhr = 0.0;
   }
   const double cl = dsqrt(g * hl);
   const double cr = dsqrt(g * hr);
@@ -462,23 +476,25 @@ AGX_HD void central_flux(const double ql[3], const double qr[3], double hl, doub
   if (dlt(span, eps)) {
     F.f[0] = F.f[1] = F.f[2] = 0.0;
     F.speed = 0.0;
-    F.pflux = 0.5 * g * 0.5 * (hl * hl + hr * hr);
+    F.pflux = half_g * 0.5 * (hl * hl + hr * hr);
     return;
   }
-  F.speed = dmax(smax, -smin);
+  F.speed = dmax(smax, dneg(smin));
   const double inv_span = ddiv(1.0, dmax(span, 1.0e-100));
   const double fl0 = ul * hl, fl1 = ul * uhl, fl2 = ul * vhl;
   const double fr0 = ur * hr, fr1 = ur * uhr, fr2 = ur * vhr;
+  const double ss = smax * smin;
+  const double fss = low_froude ? fs * ss : ss;      // fs is 1 without the scaling
   double f0 = smax * fl0 - smin * fr0;
-  f0 += (smax * smin) * (dmax(wr, ze) - dmax(wl, ze));
+  f0 += ss * (dmax(wr, ze) - dmax(wl, ze));
   f0 *= inv_span;
   double f1 = smax * fl1 - smin * fr1;
-  f1 += fs * (smax * smin) * (uhr - uhl);
+  f1 += fss * (uhr - uhl);
   f1 *= inv_span;
   double f2 = smax * fl2 - smin * fr2;
-  f2 += fs * (smax * smin) * (vhr - vhl);
+  f2 += fss * (vhr - vhl);
   f2 *= inv_span;
-  F.pflux = 0.5 * g * (smax * hl * hl - smin * hr * hr) * inv_span;
+  F.pflux = half_g * (smax * hl * hl - smin * hr * hr) * inv_span;
   const double m2 = -n2;
   F.f[0] = f0;
   F.f[1] = n1 * f1 + m2 * f2;
@@ -560,7 +576,7 @@ AGX_HD void slot_flux(const Params& P, int k, int i, const int4& c, const double
   const double hr = dmax(hre + zr - z_half, 0.0);
   FluxOut F;
   central_flux(ql, qr, hl, hr, hle, hre, normals[2 * ki], normals[2 * ki + 1], P.epsilon, z_half,
-               P.g, P.low_froude, F);
+               P.g, P.half_g, P.low_froude, F);
   if (rw_id > 0) {
     const double* hp = RW.hyd + (size_t)RW.row[rw_id - 1] * RW.ncol;
     const double wh = fmax(RW.elevation[rw_id - 1] - fmin(zl, zr), 0.0);
@@ -582,6 +598,9 @@ struct CellFlux {
   double bflux;          // contribution to boundary_flux_sum
 };
 
+// SCALED: R[i].f holds the slot's contribution -f * length already (formed
+// once for the two cells of an edge), otherwise the flux f.
+template <bool SCALED = false>
 AGX_HD void accum_cell(const Params& P, int k, const int4& c, const SlotResult R[3], const double* he,
                        const double* ze, const double* hc_arr, const double* zc_arr,
                        const double* normals, const double* lengths, double inv_area,
@@ -592,17 +611,17 @@ AGX_HD void accum_cell(const Params& P, int k, const int4& c, const SlotResult R
   for (int i = 0; i < 3; i++) {
     const int ki = 3 * k + i;
     const double len = lengths[ki];
-    const double e0 = -R[i].f[0] * len;
-    const double e1 = -R[i].f[1] * len;
-    const double e2 = -R[i].f[2] * len;
+    const double e0 = SCALED ? R[i].f[0] : -R[i].f[0] * len;
+    const double e1 = SCALED ? R[i].f[1] : -R[i].f[1] * len;
+    const double e2 = SCALED ? R[i].f[2] : -R[i].f[2] * len;
     const double hle = he[ki];
     const double zl = ze[ki];
     const double hl = R[i].hleft;
-    const double pg = len * (-P.g * 0.5 * (hl * hl - hle * hle - (hle + hc) * (zl - zc)) + R[i].pflux);
+    const double pg = len * (-P.half_g * (hl * hl - hle * hle - (hle + hc) * (zl - zc)) + R[i].pflux);
     if (full == 1 && dgt(R[i].speed, P.epsilon)) smax = dmax(smax, R[i].speed);
-    sw += e0;
-    sx += e1;
-    sy += e2;
+    sw = i == 0 ? dplus0(e0) : sw + e0;
+    sx = i == 0 ? dplus0(e1) : sx + e1;
+    sy = i == 0 ? dplus0(e2) : sy + e2;
     const int n = (i == 0) ? c.x : (i == 1) ? c.y : c.z;
     if (((n < 0) & (full == 1)) | ((n >= 0) && ((full == 1) & (full_of_neighbour[i] == 0)))) bflux += e0;
     sx -= normals[2 * ki] * pg;
@@ -710,10 +729,23 @@ AGX_HD void boundary_value(int kind, double n1, double n2, double we, double uhe
 }
 
 // ---- friction + update + fix negative -------------------------------------
+// Cube root of a positive number: y from FP32, then the series of
+// y (1 - e)^(-1/3), e = (h - y^3) / h, to the second order (e is a few 2^-24, the third
+// term below 2^-68).  y^2 is exact and the fused multiply-add leaves h - y^3
+// with one rounding, so the result is within an ulp, with five operations on
+// the FP64 pipe.
+AGX_HD double dcbrt(double h) {
+  const int64_t e16 = dbits(h) >> 52;
+  if (e16 < 1023 - 100 || e16 > 1023 + 100) return cbrt(h);
+  const double y = f2d_bits(cbrtf(cut_to_float(h)));
+  const double e = ddiv(fma(dneg(y * y), y, h), h);
+  return fma(y * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), y);
+}
+
 // h^(7/3) of the Manning term as h^2 * cbrt(h): within 3 ulp of the
 // correctly rounded power (the reference's pow(h, 7.0/3.0) is within 1),
 // at a fraction of pow's cost on the FP64 pipe.
-AGX_HD double h_pow_7_3(double h) { return (h * h) * cbrt(h); }
+AGX_HD double h_pow_7_3(double h) { return (h * h) * dcbrt(h); }
 
 AGX_HD double manning_S(const Params& P, double w, double z, double uh, double vh, double eta) {
   const double mom = dsqrt((uh * uh + vh * vh));
@@ -753,15 +785,29 @@ AGX_HD double manning_S_sloped(const Params& P, double w, const double* zv3, con
 // Quantity.update for one cell; returns false on a non-positive denominator.
 AGX_HD bool update_quantity(double& q, double expl, double& semi, double dt) {
   const double x = q;
-  double s = semi;
-  if (!dnz(x)) s = 0.0;
-  else if (dnz(s)) s = ddiv(s, x);         // 0/x is a zero: the denominator below is then exactly 1
+  const double s = semi;
   q = q + dt * expl;
-  const double den = 1.0 - dt * s;
   semi = 0.0;
+  if (!dnz(x) || !dnz(s)) return true;     // 0/x is a zero, and the denominator 1 - dt * 0 exactly 1
+  const double den = 1.0 - dt * ddiv(s, x);
   if (dle0(den)) return false;
   if (dbits(den) != dbits(1.0)) q = ddiv(q, den);
   return true;
+}
+
+// 0.5 a + 0.5 b with one addition (half_sum's bits; two zeros directly).
+AGX_HD double dhalf_sum(double a, double b) {
+  if (!dnz(a) && !dnz(b)) {
+    const int64_t z = dbits(a) & dbits(b);       // -0 only from two of them
+    double r;
+#ifdef __CUDA_ARCH__
+    r = __longlong_as_double(z);
+#else
+    memcpy(&r, &z, sizeof r);
+#endif
+    return r;
+  }
+  return half_sum(a, b);
 }
 
 }  // namespace agx
