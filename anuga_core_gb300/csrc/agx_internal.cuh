@@ -39,11 +39,7 @@ enum ErrorBits { ERR_NUMERIC = 1, ERR_TIMESTEP = 2, ERR_OVERSHOOT = 4, ERR_NAN =
 
 // A double that is NaN or an infinity (biased exponent all ones), tested on
 // the high word with integer operations.
-__host__ __device__ inline bool nonfinite64(double x) {
-  long long b;
-  memcpy(&b, &x, 8);
-  return ((b >> 52) & 0x7ff) == 0x7ff;
-}
+__host__ __device__ inline bool nonfinite64(double x) { return ((bits_of(x) >> 52) & 0x7ff) == 0x7ff; }
 // hard cap on the steps one agx_advance call may take on the device
 constexpr long long MAX_STEPS_PER_CALL = 20000000;
 

@@ -19,9 +19,11 @@
 
 namespace agx {
 
+// (as two 32-bit words on the device: masks on the whole word become FP64
+// absolute values and comparisons)
 AGX_BITS uint64_t bits_of(double x) {
 #ifdef __CUDA_ARCH__
-  return (uint64_t)__double_as_longlong(x);
+  return ((uint64_t)(uint32_t)__double2hiint(x) << 32) | (uint32_t)__double2loint(x);
 #else
   uint64_t b;
   memcpy(&b, &x, 8);
@@ -30,7 +32,7 @@ AGX_BITS uint64_t bits_of(double x) {
 }
 AGX_BITS double double_of(uint64_t b) {
 #ifdef __CUDA_ARCH__
-  return __longlong_as_double((long long)b);
+  return __hiloint2double((int)(b >> 32), (int)(uint32_t)b);
 #else
   double x;
   memcpy(&x, &b, 8);

@@ -56,15 +56,7 @@ namespace agx {
 // strictly with x, except that -0 (key -1) sorts just below +0 (key 0); the
 // comparisons treat the two zeros as equal, as IEEE comparison does.  For a
 // pair of opposite zeros dmax returns +0 and dmin -0.
-AGX_HD int64_t dbits(double x) {
-#ifdef __CUDA_ARCH__
-  return __double_as_longlong(x);
-#else
-  int64_t b;
-  memcpy(&b, &x, sizeof b);
-  return b;
-#endif
-}
+AGX_HD int64_t dbits(double x) { return (int64_t)soft64::bits(x); }
 AGX_HD int64_t dkey(double x) {
   const int64_t b = dbits(x);
   return b ^ (int64_t)((uint64_t)(b >> 63) >> 1);
@@ -798,14 +790,7 @@ AGX_HD bool update_quantity(double& q, double expl, double& semi, double dt) {
 // 0.5 a + 0.5 b with one addition (half_sum's bits; two zeros directly).
 AGX_HD double dhalf_sum(double a, double b) {
   if (!dnz(a) && !dnz(b)) {
-    const int64_t z = dbits(a) & dbits(b);       // -0 only from two of them
-    double r;
-#ifdef __CUDA_ARCH__
-    r = __longlong_as_double(z);
-#else
-    memcpy(&r, &z, sizeof r);
-#endif
-    return r;
+    return soft64::from_bits((uint64_t)(dbits(a) & dbits(b)));       // -0 only from two of them
   }
   return half_sum(a, b);
 }

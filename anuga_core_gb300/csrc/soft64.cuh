@@ -46,9 +46,14 @@ constexpr uint64_t HIDDEN = 0x0010000000000000ull;
 constexpr uint64_t QUIET = 0x0008000000000000ull;
 constexpr uint64_t DEFAULT_NAN = 0x7ff8000000000000ull;
 
+// On the device the 64 bits are taken and put together as two 32-bit words: a
+// sign or exponent mask on the whole word is turned into an FP64 absolute
+// value or comparison by the compiler (two FP64 instructions a division and a
+// square root, counted with sm__thread_inst_executed_pipe_fp64), which is the
+// pipe these functions keep free.
 SF_HD uint64_t bits(double x) {
 #ifdef __CUDA_ARCH__
-  return (uint64_t)__double_as_longlong(x);
+  return ((uint64_t)(uint32_t)__double2hiint(x) << 32) | (uint32_t)__double2loint(x);
 #else
   uint64_t b;
   memcpy(&b, &x, 8);
@@ -57,7 +62,7 @@ SF_HD uint64_t bits(double x) {
 }
 SF_HD double from_bits(uint64_t b) {
 #ifdef __CUDA_ARCH__
-  return __longlong_as_double((long long)b);
+  return __hiloint2double((int)(b >> 32), (int)(uint32_t)b);
 #else
   double x;
   memcpy(&x, &b, 8);
@@ -198,7 +203,9 @@ SF_HD uint64_t mul_bits(uint64_t a, uint64_t b) {
 // result is within a few units of its last place; the quotient built from it
 // is corrected exactly by its remainder.
 // FP32 seeds, rounded to nearest whatever the build's FP32 division and
-// square root flags (fast approximations, flush to zero) say
+// square root flags (fast approximations, flush to zero) say.  The integers
+// around them are converted as 32-bit words: conversions of 64-bit integers
+// run on the FP64 pipe.
 SF_HD float recip_rn(float x) {
 #ifdef __CUDA_ARCH__
   return __frcp_rn(x);
@@ -215,8 +222,8 @@ SF_HD float sqrt_rn(float x) {
 }
 
 SF_HD uint64_t recip64(uint64_t d) {
-  const float x = (float)(d >> 40) * (1.0f / 8388608.0f);            // d / 2^63 in [1, 2)
-  uint64_t r = (uint64_t)(recip_rn(x) * 2147483520.0f) << 33;        // ~ 2^64 / x, below 2^64
+  const float x = (float)(uint32_t)(d >> 40) * (1.0f / 8388608.0f);  // d / 2^63 in [1, 2)
+  uint64_t r = (uint64_t)(uint32_t)(recip_rn(x) * 2147483520.0f) << 33;   // ~ 2^64 / x, below 2^64
   for (int it = 0; it < 2; it++) {
     const uint64_t t = mulhi64(d, r);            // ~ d r / 2^64 ~ 2^63
     if (t <= (1ull << 63)) r += mulhi64(r, ((1ull << 63) - t) << 1);
@@ -277,8 +284,8 @@ SF_HD uint64_t div_bits(uint64_t a, uint64_t b) {
 // y ~ 2^62 / sqrt(s / 2^64) for s in [2^62, 2^64): an FP32 seed refined by two
 // Newton-Raphson steps y <- y + y (1 - x y^2) / 2 in fixed point.
 SF_HD uint64_t rsqrt64(uint64_t s) {
-  const float x = (float)(s >> 40) * (1.0f / 16777216.0f);          // s / 2^64 in [1/4, 1)
-  uint64_t y = (uint64_t)(recip_rn(sqrt_rn(x)) * 1073741824.0f) << 32;   // ~ 2^62 / sqrt(x), at most 2^63
+  const float x = (float)(uint32_t)(s >> 40) * (1.0f / 16777216.0f);   // s / 2^64 in [1/4, 1)
+  uint64_t y = (uint64_t)(uint32_t)(recip_rn(sqrt_rn(x)) * 1073741824.0f) << 32;   // ~ 2^62 / sqrt(x), at most 2^63
   for (int it = 0; it < 2; it++) {
     const uint64_t t = mulhi64(s, mulhi64(y, y));    // ~ x y^2 * 2^60
     if (t <= (1ull << 60)) y += mulhi64(y, ((1ull << 60) - t) << 3);
