@@ -198,154 +198,130 @@ SF_HD uint64_t mul_bits(uint64_t a, uint64_t b) {
   return round_pack(sign, ea + eb - 1022, sig);
 }
 
-// r ~ 2^127 / d for d in [2^63, 2^64): a 23-bit FP32 seed refined by two
-// Newton-Raphson steps r <- r + r (1 - d r / 2^127) in fixed point.  The
-// result is within a few units of its last place; the quotient built from it
-// is corrected exactly by its remainder.
-// FP32 seeds, rounded to nearest whatever the build's FP32 division and
-// square root flags (fast approximations, flush to zero) say.  The integers
-// around them are converted as 32-bit words: conversions of 64-bit integers
-// run on the FP64 pipe.
-SF_HD float recip_rn(float x) {
+// FP32 approximations of 1 / x, sqrt(x) and 1 / sqrt(x) for the digits below
+// (a few units in the last place are enough), conversions to the nearest
+// integer and of 32-bit integers only: conversions of 64-bit integers run on
+// the FP64 pipe.
+SF_HD float recip_approx(float x) {
 #ifdef __CUDA_ARCH__
-  return __frcp_rn(x);
+  return __fdividef(1.0f, x);
 #else
   return 1.0f / x;
 #endif
 }
-SF_HD float sqrt_rn(float x) {
+SF_HD float rsqrt_approx(float x) {
 #ifdef __CUDA_ARCH__
-  return __fsqrt_rn(x);
+  return rsqrtf(x);
 #else
-  return sqrtf(x);
+  return 1.0f / sqrtf(x);
+#endif
+}
+SF_HD int nearest_int(float x) {
+#ifdef __CUDA_ARCH__
+  return __float2int_rn(x);
+#else
+  return (int)lrintf(x);
 #endif
 }
 
-SF_HD uint64_t recip64(uint64_t d) {
-  const float x = (float)(uint32_t)(d >> 40) * (1.0f / 8388608.0f);  // d / 2^63 in [1, 2)
-  uint64_t r = (uint64_t)(uint32_t)(recip_rn(x) * 2147483520.0f) << 33;   // ~ 2^64 / x, below 2^64
-  for (int it = 0; it < 2; it++) {
-    const uint64_t t = mulhi64(d, r);            // ~ d r / 2^64 ~ 2^63
-    if (t <= (1ull << 63)) r += mulhi64(r, ((1ull << 63) - t) << 1);
-    else r -= mulhi64(r, (t - (1ull << 63)) << 1);
-  }
-  return r;
+// What the integer forms below do not take (NaNs, infinities, subnormal
+// operands or results, negative roots), out of line.
+#ifdef __CUDACC__
+#define SF_COLD static __host__ __device__ __noinline__
+#else
+#define SF_COLD static __attribute__((noinline))
+#endif
+SF_COLD double div_rare(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __ddiv_rn(a, b);
+#else
+  return a / b;
+#endif
+}
+SF_COLD double sqrt_rare(double a) {
+#ifdef __CUDA_ARCH__
+  return __dsqrt_rn(a);
+#else
+  return ::sqrt(a);
+#endif
 }
 
-SF_HD uint64_t div_bits(uint64_t a, uint64_t b) {
-  const uint64_t sign = (a ^ b) & SIGN;
-  const uint64_t aa = a & ~SIGN, ab = b & ~SIGN;
-  if (aa >= EXP_MASK || ab >= EXP_MASK) {
-    if (aa > EXP_MASK || ab > EXP_MASK) return nan_of(a, b);
-    if (aa == EXP_MASK) return ab == EXP_MASK ? DEFAULT_NAN : (sign | EXP_MASK);   // inf / x
-    return sign;                                                                    // x / inf
-  }
-  if (ab == 0) return aa == 0 ? DEFAULT_NAN : (sign | EXP_MASK);                    // x / 0
-  if (aa == 0) return sign;
-  uint64_t ma, mb;
-  int ea, eb;
-  unpack(a, ma, ea);
-  unpack(b, mb, eb);
-  const uint64_t n = ma << 11, d = mb << 11;        // both in [2^63, 2^64)
-  const uint64_t r = recip64(d);
-  uint64_t q = mulhi64(n, r);                        // ~ 2^63 n / d, in (2^62, 2^64), a few units off
-  // the remainder R = 2^63 n - q d in 128 bits (two's complement)
-  const uint64_t nh = n >> 1, nl = (n & 1) << 63;
-  {
-    // one Newton step on the quotient, q += R / d = R r / 2^127, from the
-    // top bits of R (|R| < 2^70 here, so R >> 7 fits a signed 64-bit word)
-    const uint64_t pl = q * d, ph = mulhi64(q, d);
-    const uint64_t rl = nl - pl;
-    const uint64_t rh = nh - ph - (uint64_t)(nl < pl);
-    const int64_t v = (int64_t)((rh << 57) | (rl >> 7));
-    const uint64_t dq = mulhi64(v < 0 ? 0ull - (uint64_t)v : (uint64_t)v, r) >> 56;
-    q = v < 0 ? q - dq : q + dq;
-  }
-  // then to floor(2^63 n / d) exactly: 0 <= R < d
-  uint64_t sticky = 0;
-  for (int it = 0; it < 4; it++) {
-    const uint64_t pl = q * d, ph = mulhi64(q, d);
-    const uint64_t rl = nl - pl;
-    const uint64_t rh = nh - ph - (uint64_t)(nl < pl);
-    if ((int64_t)rh < 0) {                 // remainder negative: q too large
-      q -= 1;
-    } else if (rh != 0 || rl >= d) {       // remainder at least d: q too small
-      q += 1;
-    } else {
-      sticky = rl != 0;
-      break;
-    }
-  }
-  // the quotient is q / 2^63 * 2^(ea - eb), q's leading one at bit 63 or 62
-  if (q >> 63) return round_pack(sign, ea - eb + 1023, (q >> 1) | (q & 1) | sticky);
-  return round_pack(sign, ea - eb + 1022, q | sticky);
+// The 55-bit value q in [2^54, 2^55) with its low bit set for anything below,
+// rounded to 53 bits and packed with biased exponent e (1 .. 2046).
+SF_HD double pack55(uint64_t sign, int e, uint64_t q) {
+  const uint64_t r = (q + 1 + ((q >> 2) & 1)) >> 2;      // to nearest, ties to even
+  return from_bits(sign | (((uint64_t)(uint32_t)(e - 1) << 52) + r));
 }
 
-// y ~ 2^62 / sqrt(s / 2^64) for s in [2^62, 2^64): an FP32 seed refined by two
-// Newton-Raphson steps y <- y + y (1 - x y^2) / 2 in fixed point.
-SF_HD uint64_t rsqrt64(uint64_t s) {
-  const float x = (float)(uint32_t)(s >> 40) * (1.0f / 16777216.0f);   // s / 2^64 in [1/4, 1)
-  uint64_t y = (uint64_t)(uint32_t)(recip_rn(sqrt_rn(x)) * 1073741824.0f) << 32;   // ~ 2^62 / sqrt(x), at most 2^63
-  for (int it = 0; it < 2; it++) {
-    const uint64_t t = mulhi64(s, mulhi64(y, y));    // ~ x y^2 * 2^60
-    if (t <= (1ull << 60)) y += mulhi64(y, ((1ull << 60) - t) << 3);
-    else y -= mulhi64(y, (t - (1ull << 60)) << 3);
+// a / b by three digits of the quotient n / d in [1, 2) (n, d the
+// significands): each digit is the nearest integer to the FP32 quotient of the remainder's
+// leading 31 bits and d, scaled by 2^17, 2^18 and 2^19.  The FP32 relative
+// error is below 2^-21 (d's cut 2^-30, reciprocal, product and conversion 2^-22.4
+// together), so a digit is off by less than 0.5 + 2^-2 of the scaled quotient,
+// the remainders (exact in 64-bit wrap-around arithmetic) stay below d in
+// magnitude, the next digits below 2^19, and the last remainder gives the
+// floor after one correction and the sticky bit.
+SF_HD double div(double a, double b) {
+  const uint64_t ua = bits(a), ub = bits(b);
+  const uint64_t sign = (ua ^ ub) & SIGN;
+  const int ea = (int)((uint32_t)(ua >> 52) & 0x7ffu), eb = (int)((uint32_t)(ub >> 52) & 0x7ffu);
+  uint64_t n = (ua & FRAC) | HIDDEN;
+  const uint64_t d = (ub & FRAC) | HIDDEN;
+  const int less = n < d ? 1 : 0;
+  const int e = ea - eb + 1023 - less;
+  if ((unsigned)(eb - 1) >= 2046u || (unsigned)(ea - 1) >= 2046u || (unsigned)(e - 1) >= 2046u) {
+    if ((ua << 1) == 0 && (unsigned)(eb - 1) < 2046u) return from_bits(sign);      // 0 / x
+    return div_rare(a, b);
   }
-  return y;
+  n <<= less;
+  const float r = recip_approx((float)(int)(uint32_t)(d >> 22));                 // 2^22 / d
+  const int q1 = nearest_int((float)(int)(uint32_t)(n >> 23) * (r * 262144.0f));  // n / d * 2^17
+  int64_t rem = (int64_t)((n << 17) - (uint64_t)(uint32_t)q1 * d);
+  const int q2 = nearest_int((float)(int)(rem >> 23) * (r * 524288.0f));          // rem / d * 2^18
+  rem = (int64_t)(((uint64_t)rem << 18) - (uint64_t)(int64_t)q2 * d);
+  const int q3 = nearest_int((float)(int)(rem >> 23) * (r * 1048576.0f));         // rem / d * 2^19
+  rem = (int64_t)(((uint64_t)rem << 19) - (uint64_t)(int64_t)q3 * d);
+  uint64_t q = ((uint64_t)(uint32_t)q1 << 37) + ((uint64_t)(int64_t)q2 << 19) + (uint64_t)(int64_t)q3;
+  const bool low = rem < 0;                       // floor
+  q -= low ? 1 : 0;
+  rem += low ? (int64_t)d : 0;
+  return pack55(sign, e, q | (rem != 0 ? 1u : 0u));
 }
 
-SF_HD uint64_t sqrt_bits(uint64_t a) {
-  const uint64_t aa = a & ~SIGN;
-  if (aa > EXP_MASK) return a | QUIET;                  // NaN
-  if (aa == 0) return a;                                // +0, -0
-  if (a & SIGN) return DEFAULT_NAN;                     // negative
-  if (aa == EXP_MASK) return a;                         // +inf
-  uint64_t m;
-  int e;
-  unpack(a, m, e);
-  int k = e - 1023;                                     // a = (m / 2^52) 2^k
-  uint64_t s = m << 10;                                 // s / 2^62 = m / 2^52, in [1, 2)
-  if (k & 1) {                                          // an even power of two
-    s <<= 1;
-    k -= 1;
+// sqrt(a): s in [2^52, 2^54) is the significand at an even exponent; the root
+// of s is taken to 27 bits in FP32 (off by less than 2^6) and refined by two
+// digits d = remainder / (2 root), of 13 and 15 more bits, to the nearest
+// integer, with exact remainders (s scaled minus root squared): after the
+// first the root is off by less than 1 (digit below 2^19, FP32 relative
+// error below 2^-20, second-order term d^2 / (2 root) below 2^-4), after the
+// second likewise, and one correction gives the floor and the sticky bit.
+SF_HD double sqrt(double a) {
+  const uint64_t ua = bits(a);
+  const int ea = (int)(uint32_t)(ua >> 52);              // the sign too: negative operands are rare
+  if ((unsigned)(ea - 1) >= 2046u) {
+    if ((ua << 1) == 0) return a;                        // +0, -0
+    return sqrt_rare(a);
   }
-  // sqrt(a) = sqrt(s * 2^62) / 2^62 * 2^(k/2); r = floor(sqrt(s * 2^62)) in [2^62, 2^63)
-  const uint64_t y = rsqrt64(s);
-  uint64_t r = mulhi64(s, y) << 1;                      // a few units off
-  const uint64_t nh = s >> 2, nl = s << 62;             // s * 2^62
-  {
-    // one Newton step, r += R / (2 r) = R y / 2^126 with R = s 2^62 - r^2
-    // (|R| < 2^70 here: R >> 7 fits a signed 64-bit word)
-    const uint64_t ql = r * r, qh = mulhi64(r, r);
-    const uint64_t rl = nl - ql;
-    const uint64_t rh = nh - qh - (uint64_t)(nl < ql);
-    const int64_t v = (int64_t)((rh << 57) | (rl >> 7));
-    const uint64_t dr = mulhi64(v < 0 ? 0ull - (uint64_t)v : (uint64_t)v, y) >> 55;
-    r = v < 0 ? r - dr : r + dr;
-  }
-  uint64_t sticky = 0;
-  for (int it = 0; it < 4; it++) {
-    const uint64_t ql = r * r, qh = mulhi64(r, r);
-    if (qh > nh || (qh == nh && ql > nl)) {             // r^2 above: too large
-      r -= 1;
-      continue;
-    }
-    const uint64_t tl = ql + 2 * r + 1;                 // (r + 1)^2
-    const uint64_t th = qh + (uint64_t)(tl < ql);
-    if (th < nh || (th == nh && tl <= nl)) {            // (r + 1)^2 not above: too small
-      r += 1;
-      continue;
-    }
-    sticky = (qh != nh || ql != nl);
-    break;
-  }
-  return round_pack(0, k / 2 + 1023, r | sticky);
+  const int odd = (ea & 1) ^ 1;                          // ea - 1023 odd
+  const uint64_t s = ((ua & FRAC) | HIDDEN) << odd;
+  const float x = (float)(int)(uint32_t)(s >> 24);       // s / 2^24, below 2^30
+  const float y = rsqrt_approx(x);                       // 2^12 / sqrt(s)
+  const int r0 = nearest_int(x * y * 4096.0f);           // sqrt(s): 2^26 .. 2^27
+  int64_t rem = (int64_t)(s - (uint64_t)(uint32_t)r0 * (uint32_t)r0);
+  const int d1 = nearest_int((float)(int)(rem >> 4) * (y * 16.0f));      // rem 2^13 / (2 r0)
+  const uint64_t r1 = ((uint64_t)(uint32_t)r0 << 13) + (uint64_t)(int64_t)d1;
+  rem = (int64_t)(((uint64_t)rem << 26) - (r1 + ((uint64_t)(uint32_t)r0 << 13)) * (uint64_t)(int64_t)d1);
+  const int d2 = nearest_int((float)(int)(rem >> 13) * (y * 4.0f));      // rem 2^15 / (2 r1)
+  const uint64_t r2 = (r1 << 15) + (uint64_t)(int64_t)d2;
+  rem = (int64_t)(((uint64_t)rem << 30) - (r2 + (r1 << 15)) * (uint64_t)(int64_t)d2);
+  uint64_t q = r2;
+  const bool low = rem < 0;
+  q -= low ? 1 : 0;
+  return pack55(0, ((ea - 1023 - odd) >> 1) + 1023, q | (rem != 0 ? 1u : 0u));
 }
 
 SF_HD double add(double a, double b) { return from_bits(add_bits(bits(a), bits(b))); }
 SF_HD double sub(double a, double b) { return from_bits(sub_bits(bits(a), bits(b))); }
 SF_HD double mul(double a, double b) { return from_bits(mul_bits(bits(a), bits(b))); }
-SF_HD double div(double a, double b) { return from_bits(div_bits(bits(a), bits(b))); }
-SF_HD double sqrt(double a) { return from_bits(sqrt_bits(bits(a))); }
 
 }  // namespace soft64
