@@ -23,17 +23,15 @@ namespace agx {
 // blocks of a mesh of some tens of thousands of cells spread evenly over the
 // 152 SMs (40,000 cells: 157 blocks of 256 gave five SMs twice the work).
 constexpr int TPB = 128;
-// resident blocks per SM asked of the compiler for the extrapolation, flux
-// and accumulation kernels (register budgets): 64 registers for the
-// extrapolation and the flux; the accumulation keeps its own budget
+// resident blocks of 128 per SM asked of the compiler (register budgets): 64
+// registers for the extrapolation, the flux and the update, and for the
+// accumulation on large meshes (8577 against 8616 us a 4.0M-triangle run with
+// 80, 10 blocks of the extrapolation 8590, 6 of the flux 8645)
 #ifndef AGX_MINB_EXTRAP
 #define AGX_MINB_EXTRAP 8
 #endif
 #ifndef AGX_MINB_FLUX
 #define AGX_MINB_FLUX 8
-#endif
-#ifndef AGX_MINB_ACCUM
-#define AGX_MINB_ACCUM 5
 #endif
 #ifndef AGX_MINB_UPDATE
 #define AGX_MINB_UPDATE 8
@@ -148,7 +146,7 @@ __global__ void k_prep(Dev d, int mode) {
 // 465 and 439 us).
 constexpr int XCELLS = 32;
 constexpr int XTPB = 4 * XCELLS;
-template <bool VERT>
+template <bool VERT, bool IM>
 __global__ void __launch_bounds__(XTPB, AGX_MINB_EXTRAP) k_extrap(Dev d) {
   __shared__ double s_factor[XCELLS];
   __shared__ double s_h[3][XCELLS];
@@ -206,7 +204,7 @@ __global__ void __launch_bounds__(XTPB, AGX_MINB_EXTRAP) k_extrap(Dev d) {
     if (!factor0) f = wet_dry_factor(P, hk, hlo, dmax(dmax(h0, dmax(h1, h2)), hk));
     s_factor[lane] = f;
   }
-  if (grad) edge_jumps(qc, q0, q1, q2, G, jump, lo, hi);
+  if (grad) edge_jumps<IM>(qc, q0, q1, q2, G, jump, lo, hi);
   __syncthreads();
   E[0] = E[1] = E[2] = qc;
   if (grad) {
@@ -320,7 +318,7 @@ __device__ __noinline__ void stage_boundary(const Dev& d, int m, double frac) {
 // Edge fluxes.  BC: in the step loop each boundary edge's values are formed
 // by the thread that reads them.  The first thread clears the accumulators
 // of the accumulation that follows.
-template <bool BC>
+template <bool BC, bool IM>
 __global__ void __launch_bounds__(TPB, AGX_MINB_FLUX) k_flux(const __grid_constant__ Dev d, double frac) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e == 0) {
@@ -338,12 +336,13 @@ __global__ void __launch_bounds__(TPB, AGX_MINB_FLUX) k_flux(const __grid_consta
   const Riverwall RW = {d.rw_counter, d.rw_elev, d.rw_row, d.rw_hyd, d.rw_ncol};
   SlotResult R;
   double hr;
-  slot_flux(d.P, k, i, cn, d.we, d.uhe, d.vhe, d.ze, d.he, d.wb, d.uhb, d.vhb, d.normals, d.w,
+  slot_flux<IM>(d.P, k, i, cn, d.we, d.uhe, d.vhe, d.ze, d.he, d.wb, d.uhb, d.vhb, d.normals, d.w,
             d.h, d.z, RW, R, hr);
   // the contributions -f * length of the edge's two cells (opposite but for
   // the length, which a table could hold differently for the two sides)
   const double len = d.lengths[s];
-  const double e0 = dneg(R.f[0]) * len, e1 = dneg(R.f[1]) * len, e2 = dneg(R.f[2]) * len;
+  const double e0 = imul<IM>(dneg(R.f[0]), len), e1 = imul<IM>(dneg(R.f[1]), len),
+               e2 = imul<IM>(dneg(R.f[2]), len);
   d.sl0[s] = e0;
   d.sl1[s] = e1;
   d.sl2[s] = e2;
@@ -364,7 +363,8 @@ __global__ void __launch_bounds__(TPB, AGX_MINB_FLUX) k_flux(const __grid_consta
 }
 
 // timestep: form the step's timestep once every block is done.
-__global__ void __launch_bounds__(TPB, AGX_MINB_ACCUM) k_accum(Dev d, int substep, int timestep) {
+template <bool IM>
+__global__ void __launch_bounds__(TPB, IM ? 8 : 5) k_accum(Dev d, int substep, int timestep) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long key = 0ull;
   double bflux = 0.0;
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(TPB, AGX_MINB_ACCUM) k_accum(Dev d, int subste
       F.smax = 0.0;
       F.bflux = 0.0;
     } else {
-      accum_cell<true>(d.P, k, c, R, d.he, d.ze, d.h, d.z, d.normals, d.lengths, d.inv_area[k], fn, F);
+      accum_cell<true, IM>(d.P, k, c, R, d.he, d.ze, d.h, d.z, d.normals, d.lengths, d.inv_area[k], fn, F);
     }
     d.xw[k] = F.ew;
     d.xuh[k] = F.euh;
@@ -669,6 +669,8 @@ __global__ void k_clock(Dev d, cudaGraphConditionalHandle handle, int set_cond) 
 
 // ---------------------------------------------------------------------------
 static inline int nblk(int n) { return (n + TPB - 1) / TPB; }
+// Meshes from here on take the integer products (see imul).
+constexpr int IMUL_MIN_CELLS = 60000;
 static inline int xblk(int n) { return (n + XCELLS - 1) / XCELLS; }
 
 #define LAUNCHK(cat, ...)                  \
@@ -681,13 +683,30 @@ static inline int xblk(int n) { return (n + XCELLS - 1) / XCELLS; }
   } while (0)
 #define LAUNCH(...) LAUNCHK(PH_SMALL, __VA_ARGS__)
 
+template <bool VERT>
+static cudaError_t launch_extrap(const Dev& d, cudaStream_t st) {
+  if (d.N < IMUL_MIN_CELLS) LAUNCHK(PH_EXTRAP, k_extrap<VERT, false><<<xblk(d.N), XTPB, 0, st>>>(d));
+  else LAUNCHK(PH_EXTRAP, k_extrap<VERT, true><<<xblk(d.N), XTPB, 0, st>>>(d));
+  return cudaSuccess;
+}
+template <bool BC>
+static cudaError_t launch_flux(const Dev& d, cudaStream_t st, double frac) {
+  if (d.N < IMUL_MIN_CELLS) LAUNCHK(PH_FLUX, k_flux<BC, false><<<nblk(d.E), TPB, 0, st>>>(d, frac));
+  else LAUNCHK(PH_FLUX, k_flux<BC, true><<<nblk(d.E), TPB, 0, st>>>(d, frac));
+  return cudaSuccess;
+}
+static cudaError_t launch_accum(const Dev& d, cudaStream_t st, int substep, int timestep) {
+  if (d.N < IMUL_MIN_CELLS) LAUNCHK(PH_ACCUM, k_accum<false><<<nblk(d.N), TPB, 0, st>>>(d, substep, timestep));
+  else LAUNCHK(PH_ACCUM, k_accum<true><<<nblk(d.N), TPB, 0, st>>>(d, substep, timestep));
+  return cudaSuccess;
+}
+
 cudaError_t enqueue_distribute(Scenario* s, cudaStream_t st, bool with_protect, bool vertices) {
   const Dev& d = s->d;
   if (d.N == 0) return cudaSuccess;
   LAUNCHK(PH_PREP, k_prep<<<nblk(d.N), TPB, 0, st>>>(d, with_protect ? 0 : 2));
-  if (vertices) LAUNCHK(PH_EXTRAP, k_extrap<true><<<xblk(d.N), XTPB, 0, st>>>(d));
-  else LAUNCHK(PH_EXTRAP, k_extrap<false><<<xblk(d.N), XTPB, 0, st>>>(d));
-  return cudaSuccess;
+  if (vertices) return launch_extrap<true>(d, st);
+  return launch_extrap<false>(d, st);
 }
 
 cudaError_t enqueue_protect(Scenario* s, cudaStream_t st) {
@@ -706,9 +725,8 @@ cudaError_t enqueue_boundary(Scenario* s, cudaStream_t st, double t_override) {
 cudaError_t enqueue_fluxes(Scenario* s, cudaStream_t st, int substep) {
   const Dev& d = s->d;
   if (d.N == 0) return cudaSuccess;
-  LAUNCHK(PH_FLUX, k_flux<false><<<nblk(d.E), TPB, 0, st>>>(d, 0.0));
-  LAUNCHK(PH_ACCUM, k_accum<<<nblk(d.N), TPB, 0, st>>>(d, substep, 0));
-  return cudaSuccess;
+  if (cudaError_t e = launch_flux<false>(d, st, 0.0)) return e;
+  return launch_accum(d, st, substep, 0);
 }
 
 cudaError_t enqueue_forcing(Scenario* s, cudaStream_t st) {
@@ -755,7 +773,7 @@ cudaError_t enqueue_geo_transpose(Scenario* s, cudaStream_t st, const double* ro
 // a DE1 step takes 9 launches instead of 20 (DE0: 5 instead of 12).
 cudaError_t enqueue_step(Scenario* s, cudaStream_t st, unsigned long long cond_handle, bool set_cond) {
   const Dev& d = s->d;
-  const int nb = nblk(d.N), eb = nblk(d.E);
+  const int nb = nblk(d.N);
   const int stages = s->prm.timestepping_method;
   // times of the stages within the step (of time series) and how each
   // stage's update combines with the step's start (k_update's saxpy)
@@ -766,9 +784,9 @@ cudaError_t enqueue_step(Scenario* s, cudaStream_t st, unsigned long long cond_h
   LAUNCHK(PH_PREP, k_prep<<<nb, TPB, 0, st>>>(d, stages > 1 ? 1 : 0));
   for (int i = 0; i < stages; i++) {
     const bool last = i == stages - 1;
-    LAUNCHK(PH_EXTRAP, k_extrap<false><<<xblk(d.N), XTPB, 0, st>>>(d));
-    LAUNCHK(PH_FLUX, k_flux<true><<<eb, TPB, 0, st>>>(d, frac[i]));
-    LAUNCHK(PH_ACCUM, k_accum<<<nb, TPB, 0, st>>>(d, i, i == 0 ? 1 : 0));
+    if (cudaError_t e = launch_extrap<false>(d, st)) return e;
+    if (cudaError_t e = launch_flux<true>(d, st, frac[i])) return e;
+    if (cudaError_t e = launch_accum(d, st, i, i == 0 ? 1 : 0)) return e;
     if (!last) LAUNCHK(PH_UPDATE, k_update<true><<<nb, TPB, 0, st>>>(d, 1, 1, 0.0, combine[i], 0, h, sc));
     else LAUNCHK(PH_UPDATE, k_update<false><<<nb, TPB, 0, st>>>(d, 1, 1, 0.0, combine[i], s->ops.empty() ? 1 : 0, h, sc));
   }

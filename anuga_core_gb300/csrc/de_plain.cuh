@@ -89,10 +89,8 @@ AGX_HD double dplus0(double x) { return dnz(x) ? x : 0.0; }
 // AGX_INT_DIVSQRT selects, for device code, which of the two are formed with
 // integer instructions (soft64.cuh) instead of on the FP64 pipe, which bounds
 // the FP64 kernels: bit 0 division, bit 1 square root.  Measured on GB300 (152
-// SMs): 115 G divisions/s and 93 G square roots/s on the integer pipes against
-// 70 G/s each on the FP64 pipe, and a plain DE1 step of 4.0M triangles
-// 8.37 -> 6.63 ms with both (6.79 with division alone, 8.19 with the square
-// root alone).
+// SMs): 320 G divisions/s and 356 G square roots/s on the integer pipes
+// against 70 G/s each on the FP64 pipe.
 #ifndef AGX_INT_DIVSQRT
 #define AGX_INT_DIVSQRT 3
 #endif
@@ -111,6 +109,24 @@ AGX_HD double dsqrt(double x) {
 #endif
 }
 
+// A product formed with integer instructions on the device (the same bits)
+// where ON.  The extrapolation and the flux keep the FP64 pipe 76-78% busy
+// and the issue slots 16-28% on a large mesh: products moved to the integer
+// pipes run beside it until the two balance.  Per 4.0M-triangle DE1 step,
+// from 4.58 ms with none: 4.31 with the gradients' four products a quantity, the
+// eight rotations of an edge's momenta and the accumulation's normals, 4.15
+// with eight a quantity, 4.04 with 25 an edge as well (twelve a quantity 4.17:
+// past the balance; the accumulation's other products nothing on 250,000).
+// On a small mesh nothing fills the pipes and an integer product only takes
+// longer (396 cells: 840 against 974 us a run), so the kernels take a switch.
+template <bool ON>
+AGX_HD double imul(double a, double b) {
+#if defined(__CUDA_ARCH__)
+  return ON ? soft64::mul(a, b) : a * b;
+#else
+  return a * b;
+#endif
+}
 // ---- boundary kinds ------------------------------------------------------
 enum BoundaryKind : int {
   BK_NONE = 0,            // segment without a boundary object (values left as they are)
@@ -315,16 +331,19 @@ AGX_HD void limited_edges(double qc, const double jump[3], double phi, double ou
 
 // The jumps to the three edges (the auxiliary triangle's gradient over the
 // edge offsets) and the admissible jump range [lo, hi].
+template <bool IM>
 AGX_HD void edge_jumps(double qc, double q0, double q1, double q2, const double G[GEO_STRIDE], double jump[3],
                        double& lo, double& hi) {
   const double d0 = q0 - qc;
   const double d1 = q1 - q0;
   const double d2 = q2 - q0;
-  double gx = G[9] * d1 - G[8] * d2;
-  gx *= G[10];
-  double gy = G[6] * d2 - G[7] * d1;
-  gy *= G[10];
-  for (int i = 0; i < 3; i++) jump[i] = gx * G[i] + gy * G[3 + i];
+  double gx = imul<IM>(G[9], d1) - imul<IM>(G[8], d2);
+  gx = imul<IM>(gx, G[10]);
+  double gy = imul<IM>(G[6], d2) - imul<IM>(G[7], d1);
+  gy = imul<IM>(gy, G[10]);
+  jump[0] = imul<IM>(gx, G[0]) + gy * G[3];
+  jump[1] = imul<IM>(gx, G[1]) + gy * G[4];
+  jump[2] = gx * G[2] + gy * G[5];
   hi = dmax(dmax(d0, dmax(d0 + d1, d0 + d2)), 0.0);
   lo = dmin(dmin(d0, dmin(d0 + d1, d0 + d2)), 0.0);
 }
@@ -418,6 +437,7 @@ struct FluxOut {
   double pflux;      // pressure flux
 };
 
+template <bool IM>
 AGX_HD void central_flux(const double ql[3], const double qr[3], double hl, double hr,
                          double hle, double hre, double n1, double n2, double eps, double ze,
                          double g, double half_g, int low_froude, FluxOut& F) {
@@ -428,10 +448,10 @@ AGX_HD void central_flux(const double ql[3], const double qr[3], double hl, doub
     return;
   }
   const double wl = ql[0], wr = qr[0];
-  double uhl = n1 * ql[1] + n2 * ql[2];
-  double vhl = -n2 * ql[1] + n1 * ql[2];
-  double uhr = n1 * qr[1] + n2 * qr[2];
-  double vhr = -n2 * qr[1] + n1 * qr[2];
+  double uhl = imul<IM>(n1, ql[1]) + imul<IM>(n2, ql[2]);
+  double vhl = imul<IM>(n1, ql[2]) - imul<IM>(n2, ql[1]);
+  double uhr = imul<IM>(n1, qr[1]) + imul<IM>(n2, qr[2]);
+  double vhr = imul<IM>(n1, qr[2]) - imul<IM>(n2, qr[1]);
   double ul, vl = 0.0, ur, vr = 0.0;         // vl, vr: read by the low-Froude scaling only
   if (dgt0(hle)) {
     const double inv = ddiv(1.0, hle);
@@ -473,24 +493,23 @@ AGX_HD void central_flux(const double ql[3], const double qr[3], double hl, doub
   }
   F.speed = dmax(smax, dneg(smin));
   const double inv_span = ddiv(1.0, dmax(span, 1.0e-100));
-  const double fl0 = ul * hl, fl1 = ul * uhl, fl2 = ul * vhl;
-  const double fr0 = ur * hr, fr1 = ur * uhr, fr2 = ur * vhr;
+  const double fl0 = ul * hl, fl1 = imul<IM>(ul, uhl), fl2 = imul<IM>(ul, vhl);
+  const double fr0 = ur * hr, fr1 = imul<IM>(ur, uhr), fr2 = imul<IM>(ur, vhr);
   const double ss = smax * smin;
   const double fss = low_froude ? fs * ss : ss;      // fs is 1 without the scaling
-  double f0 = smax * fl0 - smin * fr0;
+  double f0 = imul<IM>(smax, fl0) - imul<IM>(smin, fr0);
   f0 += ss * (dmax(wr, ze) - dmax(wl, ze));
   f0 *= inv_span;
-  double f1 = smax * fl1 - smin * fr1;
+  double f1 = imul<IM>(smax, fl1) - imul<IM>(smin, fr1);
   f1 += fss * (uhr - uhl);
   f1 *= inv_span;
-  double f2 = smax * fl2 - smin * fr2;
+  double f2 = imul<IM>(smax, fl2) - imul<IM>(smin, fr2);
   f2 += fss * (vhr - vhl);
   f2 *= inv_span;
   F.pflux = half_g * (smax * hl * hl - smin * hr * hr) * inv_span;
-  const double m2 = -n2;
   F.f[0] = f0;
-  F.f[1] = n1 * f1 + m2 * f2;
-  F.f[2] = -m2 * f1 + n1 * f2;
+  F.f[1] = imul<IM>(n1, f1) - imul<IM>(n2, f2);
+  F.f[2] = imul<IM>(n2, f1) + imul<IM>(n1, f2);
 }
 
 AGX_HD void weir_adjust(FluxOut& F, double hl, double hr, double g, double weir_height,
@@ -535,6 +554,7 @@ struct SlotResult {
 
 // Flux across slot ki (cell k, edge i), evaluated from cell k's side
 // (:536-653).  Also returns h_right (the neighbour side's Audusse depth).
+template <bool IM = false>
 AGX_HD void slot_flux(const Params& P, int k, int i, const int4& c, const double* we, const double* uhe,
                       const double* vhe, const double* ze, const double* he, const double* wb,
                       const double* uhb, const double* vhb, const double* normals, const double* wc,
@@ -567,7 +587,7 @@ AGX_HD void slot_flux(const Params& P, int k, int i, const int4& c, const double
   const double hl = dmax(hle + zl - z_half, 0.0);
   const double hr = dmax(hre + zr - z_half, 0.0);
   FluxOut F;
-  central_flux(ql, qr, hl, hr, hle, hre, normals[2 * ki], normals[2 * ki + 1], P.epsilon, z_half,
+  central_flux<IM>(ql, qr, hl, hr, hle, hre, normals[2 * ki], normals[2 * ki + 1], P.epsilon, z_half,
                P.g, P.half_g, P.low_froude, F);
   if (rw_id > 0) {
     const double* hp = RW.hyd + (size_t)RW.row[rw_id - 1] * RW.ncol;
@@ -592,7 +612,7 @@ struct CellFlux {
 
 // SCALED: R[i].f holds the slot's contribution -f * length already (formed
 // once for the two cells of an edge), otherwise the flux f.
-template <bool SCALED = false>
+template <bool SCALED = false, bool IM = false>
 AGX_HD void accum_cell(const Params& P, int k, const int4& c, const SlotResult R[3], const double* he,
                        const double* ze, const double* hc_arr, const double* zc_arr,
                        const double* normals, const double* lengths, double inv_area,
@@ -616,8 +636,8 @@ AGX_HD void accum_cell(const Params& P, int k, const int4& c, const SlotResult R
     sy = i == 0 ? dplus0(e2) : sy + e2;
     const int n = (i == 0) ? c.x : (i == 1) ? c.y : c.z;
     if (((n < 0) & (full == 1)) | ((n >= 0) && ((full == 1) & (full_of_neighbour[i] == 0)))) bflux += e0;
-    sx -= normals[2 * ki] * pg;
-    sy -= normals[2 * ki + 1] * pg;
+    sx -= imul<IM>(normals[2 * ki], pg);
+    sy -= imul<IM>(normals[2 * ki + 1], pg);
   }
   out.ew = sw * inv_area;
   out.euh = sx * inv_area;

@@ -9,23 +9,23 @@
 // SMs: DFMA 525 G op/s, DDIV and DSQRT 70 G op/s), while its integer pipes
 // issue several warp instructions per clock per SM.  An exact binary64
 // operation built from 32- and 64-bit integer arithmetic therefore runs beside
-// the FP64 pipe.  Measured on the same part: division 115 G op/s and square
-// root 93 G op/s this way, faster than the FP64 pipe's; addition (276 G op/s)
-// and multiplication (384 G op/s) slower, and no faster split between the
-// two paths, since both take issue slots.  So the FP64 kernels divide and
-// take square roots with these functions and add and multiply on the pipe.  Every non-NaN result is bitwise the
-// IEEE result; tests/cpp/check_soft64.cpp checks that on the host against the
-// processor's own IEEE arithmetic.
+// the FP64 pipe.  Measured on the same part (agx_soft64_throughput): division
+// 320 G op/s and square root 356 G op/s this way; multiplication 429 against
+// the FP64 pipe's 525, and 839 with half of the products on each; addition
+// 262.  So the FP64 kernels divide and take square roots with these
+// functions, and large meshes form part of their products so.  Every non-NaN
+// result is bitwise the IEEE result; tests/cpp/check_soft64.cpp checks that on
+// the host against the processor's own IEEE arithmetic, agx_soft64_check on
+// the device against the FP64 pipe.
 //
-// Methods.  Addition and multiplication align or multiply the significands
-// exactly in 64- or 128-bit integers, keep a sticky bit for everything shifted
-// out, and round once with guard, round and sticky bits (Goldberg, "What every
-// computer scientist should know about floating-point arithmetic", 1991).
-// Division multiplies by a reciprocal seeded in FP32 and refined by
-// Newton-Raphson steps in 64-bit fixed point, then corrects the quotient by
-// its exact 128-bit remainder to the truncated quotient, whose remainder gives
-// the sticky bit; the square root likewise from an inverse square root
-// refined by Newton-Raphson steps, corrected by its exact remainder.
+// Methods.  Addition aligns the significands in 64-bit integers, multiplication
+// forms their exact product; a sticky bit stands for everything shifted out
+// and the result is rounded once with guard, round and sticky bits (Goldberg,
+// "What every computer scientist should know about floating-point
+// arithmetic", 1991).  Division and square root take a few digits guessed in
+// FP32 with exact remainders (the schoolbook digit recurrences with a large
+// radix and nearest digits), whose last remainder gives the floor and the
+// sticky bit.
 #pragma once
 #include <stdint.h>
 #include <string.h>
@@ -175,29 +175,6 @@ SF_HD uint64_t add_bits(uint64_t a, uint64_t b) {
 
 SF_HD uint64_t sub_bits(uint64_t a, uint64_t b) { return add_bits(a, b ^ SIGN); }
 
-SF_HD uint64_t mul_bits(uint64_t a, uint64_t b) {
-  const uint64_t sign = (a ^ b) & SIGN;
-  const uint64_t aa = a & ~SIGN, ab = b & ~SIGN;
-  if (aa >= EXP_MASK || ab >= EXP_MASK) {
-    if (aa > EXP_MASK || ab > EXP_MASK) return nan_of(a, b);
-    if (aa == 0 || ab == 0) return DEFAULT_NAN;     // inf * 0
-    return sign | EXP_MASK;
-  }
-  if (aa == 0 || ab == 0) return sign;
-  uint64_t ma, mb;
-  int ea, eb;
-  unpack(a, ma, ea);
-  unpack(b, mb, eb);
-  // ma * (mb << 11) lies in [2^115, 2^117): its high word has the leading
-  // one at bit 51 or 52; move it to bit 61 or 62 with the next 10 bits and a
-  // sticky bit for the rest
-  const uint64_t bb = mb << 11;
-  const uint64_t lo = ma * bb;
-  const uint64_t hi = mulhi64(ma, bb);
-  const uint64_t sig = (hi << 10) | (lo >> 54) | (uint64_t)((lo << 10) != 0);
-  return round_pack(sign, ea + eb - 1022, sig);
-}
-
 // FP32 approximations of 1 / x, sqrt(x) and 1 / sqrt(x) for the digits below
 // (a few units in the last place are enough), conversions to the nearest
 // integer and of 32-bit integers only: conversions of 64-bit integers run on
@@ -253,6 +230,47 @@ SF_HD double pack55(uint64_t sign, int e, uint64_t q) {
   return from_bits(sign | (((uint64_t)(uint32_t)(e - 1) << 52) + r));
 }
 
+SF_COLD double mul_rare(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+
+// x << s with y's top bits shifted in (0 < s < 32)
+SF_HD uint32_t shl_in(uint32_t x, uint32_t y, int s) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(y, x, s);
+#else
+  return (x << s) | (y >> (32 - s));
+#endif
+}
+
+// a * b: the exact product of the significands from four 32-bit ones.
+SF_HD double mul(double a, double b) {
+  const uint64_t ua = bits(a), ub = bits(b);
+  const uint64_t sign = (ua ^ ub) & SIGN;
+  const int ea = (int)((uint32_t)(ua >> 52) & 0x7ffu), eb = (int)((uint32_t)(ub >> 52) & 0x7ffu);
+  const int e = ea + eb - 1023;
+  if ((unsigned)(ea - 1) >= 2046u || (unsigned)(eb - 1) >= 2046u || (unsigned)(e - 1) >= 2045u) {
+    if (((ua << 1) == 0 && eb < 2047) || ((ub << 1) == 0 && ea < 2047)) return from_bits(sign);
+    return mul_rare(a, b);
+  }
+  const uint64_t x = (ua & FRAC) | HIDDEN, y = ((ub & FRAC) | HIDDEN) << 11;     // product in [2^115, 2^117)
+  const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32), y0 = (uint32_t)y, y1 = (uint32_t)(y >> 32);
+  const uint64_t p = (uint64_t)x0 * y0;
+  const uint64_t m = (uint64_t)x0 * y1 + (p >> 32);
+  const uint64_t n = (uint64_t)x1 * y0 + (uint32_t)m;
+  const uint64_t hi = (uint64_t)x1 * y1 + (m >> 32) + (n >> 32);                 // leading one at bit 51 or 52
+  const int top = (int)(hi >> 52), s = 3 - top;
+  // hi : lo shifted left by s (2 or 3): the 55 bits, and whether any are set below
+  const uint32_t h1 = (uint32_t)(hi >> 32), h0 = (uint32_t)hi, l1 = (uint32_t)n, l0 = (uint32_t)p;
+  const uint32_t q1 = shl_in(h1, h0, s), q0 = shl_in(h0, l1, s);
+  const bool below = (shl_in(l1, l0, s) | (l0 << s)) != 0;
+  return pack55(sign, e + top, ((uint64_t)q1 << 32) | q0 | (below ? 1u : 0u));
+}
+
 // a / b by three digits of the quotient n / d in [1, 2) (n, d the
 // significands): each digit is the nearest integer to the FP32 quotient of the remainder's
 // leading 31 bits and d, scaled by 2^17, 2^18 and 2^19.  The FP32 relative
@@ -273,7 +291,7 @@ SF_HD double div(double a, double b) {
     if ((ua << 1) == 0 && (unsigned)(eb - 1) < 2046u) return from_bits(sign);      // 0 / x
     return div_rare(a, b);
   }
-  n <<= less;
+  n = less ? n + n : n;
   const float r = recip_approx((float)(int)(uint32_t)(d >> 22));                 // 2^22 / d
   const int q1 = nearest_int((float)(int)(uint32_t)(n >> 23) * (r * 262144.0f));  // n / d * 2^17
   int64_t rem = (int64_t)((n << 17) - (uint64_t)(uint32_t)q1 * d);
@@ -303,7 +321,8 @@ SF_HD double sqrt(double a) {
     return sqrt_rare(a);
   }
   const int odd = (ea & 1) ^ 1;                          // ea - 1023 odd
-  const uint64_t s = ((ua & FRAC) | HIDDEN) << odd;
+  const uint64_t m = (ua & FRAC) | HIDDEN;
+  const uint64_t s = odd ? m + m : m;
   const float x = (float)(int)(uint32_t)(s >> 24);       // s / 2^24, below 2^30
   const float y = rsqrt_approx(x);                       // 2^12 / sqrt(s)
   const int r0 = nearest_int(x * y * 4096.0f);           // sqrt(s): 2^26 .. 2^27
@@ -322,6 +341,5 @@ SF_HD double sqrt(double a) {
 
 SF_HD double add(double a, double b) { return from_bits(add_bits(bits(a), bits(b))); }
 SF_HD double sub(double a, double b) { return from_bits(sub_bits(bits(a), bits(b))); }
-SF_HD double mul(double a, double b) { return from_bits(mul_bits(bits(a), bits(b))); }
 
 }  // namespace soft64
