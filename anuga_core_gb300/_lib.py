@@ -30,6 +30,7 @@ FIELD = {n: i for i, n in enumerate(FIELDS)}
 
 (BC_NONE, BC_REFLECTIVE, BC_TRANSMISSIVE, BC_TRANSMISSIVE_C, BC_DIRICHLET, BC_TIME_SERIES, BC_TRANSMISSIVE_N0,
  BC_TRANSMISSIVE_SET_STAGE, BC_TRANSMISSIVE_ZERO_MOM, BC_FLATHER, BC_CHARACTERISTIC, BC_INFLOW) = range(12)
+E_NOMEM = -3             # include/agx.h
 STOP_YIELD, STOP_FINAL, STOP_MAXSTEPS, STOP_ERROR = 1, 2, 3, 4
 PHASES = ("prep", "extrap", "bc", "flux", "accum", "update", "rate", "small")
 PHASE_COUNT = len(PHASES)
@@ -97,6 +98,8 @@ def load(path=None):
         "agx_sww_frame": ([H, ctypes.c_double, ctypes.c_int32, ctypes.POINTER(ctypes.c_float),
                            ctypes.POINTER(ctypes.c_float)], ctypes.c_int32),
         "agx_sww_frame_async": ([H, ctypes.c_double, ctypes.c_int32], ctypes.c_int32),
+        "agx_sww_frame_take": ([H, P(ctypes.POINTER(ctypes.c_float))], ctypes.c_int32),
+        "agx_frame_give": ([ctypes.POINTER(ctypes.c_float)], None),
         "agx_sww_frame_wait": ([H, P(ctypes.POINTER(ctypes.c_float)), P(ctypes.POINTER(ctypes.c_float))],
                                ctypes.c_int32),
         "agx_get_state": ([H, _f64p, _f64p, _f64p, ctypes.c_int64], ctypes.c_int32),
@@ -141,14 +144,38 @@ def load(path=None):
     return L
 
 
-def _frame_arrays(fn, args, P, N):
-    """Wait through `fn` for a frame in page-locked memory and copy it out."""
+class _Frame:
+    """A page-locked frame buffer of the library, given back when the last
+    array over it is gone."""
+
+    def __init__(self, ptr, n):
+        self.ptr = ptr
+        self.__array_interface__ = {"shape": (n,), "typestr": "<f4", "version": 3,
+                                    "data": (ctypes.cast(ptr, ctypes.c_void_p).value, False)}
+
+    def __del__(self):
+        try:
+            load().agx_frame_give(self.ptr)
+        except Exception:
+            pass
+
+
+def _frame_arrays(take, wait, args, P, N):
+    """The frame started last as (vertex [3, P], centroid [3, N]) arrays of the
+    caller's own: over the page-locked buffer the device wrote, which the
+    next frames leave alone, or copies where the callers hold too many such
+    buffers already.  (Copying 72 MB into fresh pages took 5.8 ms.)"""
     fp = ctypes.POINTER(ctypes.c_float)
-    v, c = fp(), fp()
-    check(fn(*args, ctypes.byref(v), ctypes.byref(c)))
-    vv = np.ctypeslib.as_array(v, shape=(3 * P,)).copy().reshape(3, P) if P else np.zeros((3, 0), np.float32)
-    cc = np.ctypeslib.as_array(c, shape=(3 * N,)).copy().reshape(3, N)
-    return vv, cc
+    f = fp()
+    code = take(*args, ctypes.byref(f))
+    if code == E_NOMEM:
+        v, c = fp(), fp()
+        check(wait(*args, ctypes.byref(v), ctypes.byref(c)))
+        vv = np.ctypeslib.as_array(v, shape=(3 * P,)).copy().reshape(3, P) if P else np.zeros((3, 0), np.float32)
+        return vv, np.ctypeslib.as_array(c, shape=(3 * N,)).copy().reshape(3, N)
+    check(code)
+    a = np.asarray(_Frame(f, 3 * P + 3 * N))
+    return a[:3 * P].reshape(3, P), a[3 * P:].reshape(3, N)
 
 
 def last_error():
@@ -276,8 +303,8 @@ class Scenario:
         check(self.L.agx_sww_frame_async(self.h, float(min_storable_height), 1 if centroid_averaging else 0))
 
     def sww_frame_wait(self):
-        """The frame started last, as copies of (vertex [3, P], centroid [3, N]) float32."""
-        return _frame_arrays(self.L.agx_sww_frame_wait, (self.h,), self._sww_P, self.N)
+        """The frame started last: (vertex [3, P], centroid [3, N]) float32, the caller's own."""
+        return _frame_arrays(self.L.agx_sww_frame_take, self.L.agx_sww_frame_wait, (self.h,), self._sww_P, self.N)
 
     def device_ptr(self, name):
         p = ctypes.c_void_p()

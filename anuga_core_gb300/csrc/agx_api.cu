@@ -6,6 +6,8 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <unordered_map>
+#include <unordered_set>
 
 namespace agx {
 
@@ -75,6 +77,87 @@ static agx_status fail(agx_status code, const char* fmt, ...) {
       return fail(AGX_E_CUDA, "%s failed: %s (%s:%d)", #call, cudaGetErrorString(_e),   \
                   __FILE__, __LINE__);                                                  \
   } while (0)
+
+// ---- output frame buffers ------------------------------------------------
+namespace {
+struct FrameBuffers {
+  std::mutex mu;
+  std::unordered_map<float*, size_t> size;              // every live buffer
+  std::unordered_multimap<size_t, float*> kept;
+  std::unordered_set<float*> taken;
+  size_t kept_bytes = 0, taken_bytes = 0;
+};
+// never destroyed: arrays that hold a frame may outlive the library's statics
+FrameBuffers& frame_buffers() {
+  static FrameBuffers* b = new FrameBuffers();
+  return *b;
+}
+}  // namespace
+
+cudaError_t frame_buffer_get(size_t bytes, float** out) {
+  FrameBuffers& B = frame_buffers();
+  {
+    std::lock_guard<std::mutex> lock(B.mu);
+    auto it = B.kept.find(bytes);
+    if (it != B.kept.end()) {
+      *out = it->second;
+      B.kept.erase(it);
+      B.kept_bytes -= bytes;
+      return cudaSuccess;
+    }
+  }
+  float* p = nullptr;
+  const cudaError_t e = cudaMallocHost(&p, bytes);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(B.mu);
+  B.size[p] = bytes;
+  *out = p;
+  return cudaSuccess;
+}
+
+bool frame_buffer_take(float* p) {
+  FrameBuffers& B = frame_buffers();
+  std::lock_guard<std::mutex> lock(B.mu);
+  const size_t bytes = B.size[p];
+  if (B.taken_bytes + bytes > FRAME_TAKEN) return false;
+  B.taken.insert(p);
+  B.taken_bytes += bytes;
+  return true;
+}
+
+void frame_buffer_give(float* p) {
+  FrameBuffers& B = frame_buffers();
+  {
+    std::lock_guard<std::mutex> lock(B.mu);
+    auto it = B.size.find(p);
+    if (it == B.size.end()) return;
+    const size_t bytes = it->second;
+    if (B.taken.erase(p)) B.taken_bytes -= bytes;
+    if (B.kept_bytes + bytes <= FRAME_KEEP) {
+      B.kept.emplace(bytes, p);
+      B.kept_bytes += bytes;
+      return;
+    }
+    B.size.erase(it);
+  }
+  cudaFreeHost(p);
+}
+
+void frame_buffer_release(float* p, size_t bytes) {
+  FrameBuffers& B = frame_buffers();
+  std::vector<float*> gone;
+  {
+    std::lock_guard<std::mutex> lock(B.mu);
+    if (p && B.size.erase(p)) gone.push_back(p);
+    for (auto it = B.kept.find(bytes); it != B.kept.end(); it = B.kept.find(bytes)) {
+      gone.push_back(it->second);
+      B.size.erase(it->second);
+      B.kept.erase(it);
+      B.kept_bytes -= bytes;
+    }
+  }
+  for (float* q : gone) cudaFreeHost(q);
+}
 
 static size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -334,12 +417,14 @@ agx_status agx_scenario_destroy(agx_handle h) {
     if (op.idx) cudaFree(op.idx);
   if (s->node_off) cudaFree(s->node_off);
   if (s->node_slot) cudaFree(s->node_slot);
-  if (s->frame) cudaFree(s->frame);
   if (s->copy_stream) {
     cudaStreamSynchronize(s->copy_stream);
     cudaStreamDestroy(s->copy_stream);
   }
-  if (s->frame_host) cudaFreeHost(s->frame_host);
+  if (s->frame) {
+    cudaFree(s->frame);
+    frame_buffer_release(s->frame_host, s->frame_bytes);
+  }
   if (s->frame_done) cudaEventDestroy(s->frame_done);
   if (s->frame_ready) cudaEventDestroy(s->frame_ready);
   if (s->bseries) cudaFree(s->bseries);
@@ -405,9 +490,11 @@ agx_status agx_sww_bind(agx_handle h, int64_t P, const int32_t* node_offsets, co
   if (st) return st;
   if (h->node_off) cudaFree(h->node_off);
   if (h->node_slot) cudaFree(h->node_slot);
-  if (h->frame) cudaFree(h->frame);
   if (h->copy_stream) CK(cudaStreamSynchronize(h->copy_stream));
-  if (h->frame_host) cudaFreeHost(h->frame_host);
+  if (h->frame) {
+    cudaFree(h->frame);
+    frame_buffer_release(h->frame_host, h->frame_bytes);
+  }
   if (h->frame_done) cudaEventDestroy(h->frame_done);
   if (h->frame_ready) cudaEventDestroy(h->frame_ready);
   h->node_off = h->node_slot = nullptr;
@@ -418,7 +505,8 @@ agx_status agx_sww_bind(agx_handle h, int64_t P, const int32_t* node_offsets, co
   CK(cudaMalloc(&h->node_off, (size_t)(P + 1) * 4));
   CK(cudaMalloc(&h->node_slot, (size_t)3 * h->N * 4 + 4));
   CK(cudaMalloc(&h->frame, fbytes));
-  CK(cudaMallocHost(&h->frame_host, fbytes));
+  h->frame_bytes = fbytes;
+  CK(frame_buffer_get(fbytes, &h->frame_host));
   CK(cudaEventCreateWithFlags(&h->frame_done, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&h->frame_ready, cudaEventDisableTiming));
   if (!h->copy_stream) CK(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
@@ -445,6 +533,7 @@ agx_status agx_sww_frame_async(agx_handle h, double min_storable_height, int32_t
   if (!h->frame) return fail(AGX_E_STATE, "agx_sww_bind first");
   // the frame kernels wait for the previous frame's copy to leave the buffer;
   // the copy runs on its own stream, so the steps enqueued next overlap it
+  if (!h->frame_host) CK(frame_buffer_get(h->frame_bytes, &h->frame_host));     // the last one was taken
   CK(cudaStreamWaitEvent(h->stream, h->frame_done, 0));
   CK(enqueue_sww_frame(h, h->stream, min_storable_height, centroid_averaging ? 1 : 0));
   CK(cudaEventRecord(h->frame_ready, h->stream));
@@ -455,10 +544,37 @@ agx_status agx_sww_frame_async(agx_handle h, double min_storable_height, int32_t
   return AGX_OK;
 }
 
+// The last frame in the scenario's buffer; copied again from the device if
+// that buffer has been taken since.
+static agx_status frame_on_host(agx_handle h) {
+  if (!h->frame_host) {
+    CK(frame_buffer_get(h->frame_bytes, &h->frame_host));
+    CK(cudaMemcpyAsync(h->frame_host, h->frame, ((size_t)3 * h->P + 3 * (size_t)h->N) * 4, cudaMemcpyDeviceToHost,
+                       h->copy_stream));
+    CK(cudaEventRecord(h->frame_done, h->copy_stream));
+  }
+  CK(cudaEventSynchronize(h->frame_done));
+  return AGX_OK;
+}
+
+agx_status agx_sww_frame_take(agx_handle h, float** frame) {
+  if (!h || !frame) return fail(AGX_E_INVALID, "bad arguments");
+  if (!h->frame) return fail(AGX_E_STATE, "agx_sww_bind first");
+  agx_status st = frame_on_host(h);
+  if (st) return st;
+  if (!frame_buffer_take(h->frame_host)) return fail(AGX_E_NOMEM, "callers hold 1 GiB of frames");
+  *frame = h->frame_host;
+  h->frame_host = nullptr;
+  return AGX_OK;
+}
+
+void agx_frame_give(float* frame) { frame_buffer_give(frame); }
+
 agx_status agx_sww_frame_wait(agx_handle h, const float** vertex, const float** centroid) {
   if (!h || !vertex || !centroid) return fail(AGX_E_INVALID, "bad arguments");
-  if (!h->frame_host) return fail(AGX_E_STATE, "agx_sww_bind first");
-  CK(cudaEventSynchronize(h->frame_done));
+  if (!h->frame) return fail(AGX_E_STATE, "agx_sww_bind first");
+  agx_status st = frame_on_host(h);
+  if (st) return st;
   *vertex = h->frame_host;
   *centroid = h->frame_host + 3 * (size_t)h->P;
   return AGX_OK;

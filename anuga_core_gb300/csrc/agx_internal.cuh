@@ -211,7 +211,8 @@ struct Scenario {
   int* node_off = nullptr;
   int* node_slot = nullptr;
   float* frame = nullptr;
-  float* frame_host = nullptr;           // pinned copy of the last frame (asynchronous output)
+  float* frame_host = nullptr;           // page-locked copy of the last frame (null once taken)
+  size_t frame_bytes = 0;
   cudaEvent_t frame_done = nullptr;      // recorded after that copy
   cudaEvent_t frame_ready = nullptr;     // recorded after the frame kernels
   cudaStream_t copy_stream = nullptr;    // the copy's own stream: the next steps need not wait for it
@@ -247,6 +248,18 @@ struct TraceRange {
   TraceRange& operator=(const TraceRange&) = delete;
 };
 #define AGX_TRACE(name) ::agx::TraceRange agx_trace_range_(name)
+
+// Page-locked buffers of output frames (agx_api.cu).  A buffer belongs to a
+// scenario or, once taken, to a caller; one given back is kept for the next
+// frame of its size (page-locking 72 MB takes some 20 ms), at most
+// FRAME_KEEP bytes in all, and those of a size are released with a scenario
+// of that size.
+constexpr size_t FRAME_KEEP = 256u << 20;
+constexpr size_t FRAME_TAKEN = 1u << 30;     // bytes callers may hold
+cudaError_t frame_buffer_get(size_t bytes, float** out);
+bool frame_buffer_take(float* p);            // false: the callers hold FRAME_TAKEN already
+void frame_buffer_give(float* p);
+void frame_buffer_release(float* p, size_t bytes);   // p (may be null) and the kept ones of its size
 
 // launch accounting
 void count_launch(int64_t n = 1);

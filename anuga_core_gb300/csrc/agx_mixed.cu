@@ -1356,7 +1356,8 @@ struct ScnHost {
   int* sww_off = nullptr;
   int* sww_slot = nullptr;
   float* frame = nullptr;
-  float* frame_host = nullptr;
+  float* frame_host = nullptr;            // null once taken
+  size_t frame_bytes = 0;
   cudaEvent_t frame_done = nullptr;
   cudaEvent_t frame_ready = nullptr;      // after the frame kernels
   cudaStream_t copy_stream = nullptr;     // the frame copy's own stream
@@ -1486,8 +1487,10 @@ static void free_sww(ScnHost& s) {
   }
   if (s.sww_off) cudaFree(s.sww_off);
   if (s.sww_slot) cudaFree(s.sww_slot);
-  if (s.frame) cudaFree(s.frame);
-  if (s.frame_host) cudaFreeHost(s.frame_host);
+  if (s.frame) {
+    cudaFree(s.frame);
+    frame_buffer_release(s.frame_host, s.frame_bytes);
+  }
   if (s.frame_done) cudaEventDestroy(s.frame_done);
   if (s.frame_ready) cudaEventDestroy(s.frame_ready);
   s.sww_off = s.sww_slot = nullptr;
@@ -2658,7 +2661,8 @@ agx_status agx_pool_sww_bind(agx_pool p, int32_t sid, int64_t P, const int32_t* 
   PCK(cudaMalloc(&sh.sww_off, (size_t)(P + 1) * 4));
   PCK(cudaMalloc(&sh.sww_slot, (size_t)S3 * 4 + 4));
   PCK(cudaMalloc(&sh.frame, fbytes));
-  PCK(cudaMallocHost(&sh.frame_host, fbytes));
+  sh.frame_bytes = fbytes;
+  PCK(frame_buffer_get(fbytes, &sh.frame_host));
   PCK(cudaEventCreateWithFlags(&sh.frame_done, cudaEventDisableTiming));
   PCK(cudaEventCreateWithFlags(&sh.frame_ready, cudaEventDisableTiming));
   PCK(cudaStreamCreateWithFlags(&sh.copy_stream, cudaStreamNonBlocking));
@@ -2675,6 +2679,7 @@ agx_status agx_pool_sww_frame_async(agx_pool p, int32_t sid, double min_storable
   if (!sh.frame) return pfail(AGX_E_STATE, "agx_pool_sww_bind first");
   agx_status st = ensure_work(p, sid);
   if (st) return st;
+  if (!sh.frame_host) PCK(frame_buffer_get(sh.frame_bytes, &sh.frame_host));     // the last one was taken
   cudaStream_t s = p->stream;
   // the frame kernels wait for the previous frame's copy to leave the buffer;
   // the copy runs on its own stream, so the steps enqueued next overlap it
@@ -2695,12 +2700,38 @@ agx_status agx_pool_sww_frame_async(agx_pool p, int32_t sid, double min_storable
   return AGX_OK;
 }
 
+// The last frame in the scenario's buffer; copied again from the device if
+// that buffer has been taken since.
+static agx_status frame_on_host(ScnHost& sh) {
+  if (!sh.frame_host) {
+    PCK(frame_buffer_get(sh.frame_bytes, &sh.frame_host));
+    PCK(cudaMemcpyAsync(sh.frame_host, sh.frame, ((size_t)3 * sh.sww_P + 3 * (size_t)sh.N) * 4,
+                        cudaMemcpyDeviceToHost, sh.copy_stream));
+    PCK(cudaEventRecord(sh.frame_done, sh.copy_stream));
+  }
+  PCK(cudaEventSynchronize(sh.frame_done));
+  return AGX_OK;
+}
+
+agx_status agx_pool_sww_frame_take(agx_pool p, int32_t sid, float** frame) {
+  if (!p || sid < 0 || sid >= p->cap_scn || !p->scn[sid].alive || !frame) return pfail(AGX_E_INVALID, "bad arguments");
+  ScnHost& sh = p->scn[sid];
+  if (!sh.frame) return pfail(AGX_E_STATE, "agx_pool_sww_bind first");
+  agx_status st = frame_on_host(sh);
+  if (st) return st;
+  if (!frame_buffer_take(sh.frame_host)) return pfail(AGX_E_NOMEM, "callers hold 1 GiB of frames");
+  *frame = sh.frame_host;
+  sh.frame_host = nullptr;
+  return AGX_OK;
+}
+
 agx_status agx_pool_sww_frame_wait(agx_pool p, int32_t sid, const float** vertex, const float** centroid) {
   if (!p || sid < 0 || sid >= p->cap_scn || !p->scn[sid].alive || !vertex || !centroid)
     return pfail(AGX_E_INVALID, "bad arguments");
   ScnHost& sh = p->scn[sid];
-  if (!sh.frame_host) return pfail(AGX_E_STATE, "agx_pool_sww_bind first");
-  PCK(cudaEventSynchronize(sh.frame_done));
+  if (!sh.frame) return pfail(AGX_E_STATE, "agx_pool_sww_bind first");
+  agx_status st = frame_on_host(sh);
+  if (st) return st;
   *vertex = sh.frame_host;
   *centroid = sh.frame_host + 3 * (size_t)sh.sww_P;
   return AGX_OK;

@@ -57,6 +57,7 @@ def lib():
             "agx_pool_set_fixed_flux_timestep": ([H, ctypes.c_int32, ctypes.c_double], ctypes.c_int32),
             "agx_pool_sww_bind": ([H, ctypes.c_int32, ctypes.c_int64, _i32p, _i32p], ctypes.c_int32),
             "agx_pool_sww_frame_async": ([H, ctypes.c_int32, ctypes.c_double, ctypes.c_int32], ctypes.c_int32),
+            "agx_pool_sww_frame_take": ([H, ctypes.c_int32, P(ctypes.POINTER(ctypes.c_float))], ctypes.c_int32),
             "agx_pool_sww_frame_wait": ([H, ctypes.c_int32, P(ctypes.POINTER(ctypes.c_float)),
                                          P(ctypes.POINTER(ctypes.c_float))], ctypes.c_int32),
             "agx_pool_set_clock": ([H, ctypes.c_int32, ctypes.c_double, ctypes.c_double, ctypes.c_double,
@@ -237,7 +238,8 @@ class Pool:
 
     def sww_frame_wait(self, sid, P):
         N, _ = self._keep[sid]
-        return _lib._frame_arrays(self.L.agx_pool_sww_frame_wait, (self.h, int(sid)), P, N)
+        return _lib._frame_arrays(self.L.agx_pool_sww_frame_take, self.L.agx_pool_sww_frame_wait, (self.h, int(sid)),
+                                  P, N)
 
     def set_fixed_flux_timestep(self, sid, flux_timestep):
         check(self.L.agx_pool_set_fixed_flux_timestep(self.h, int(sid), float(flux_timestep or 0.0)))

@@ -274,6 +274,13 @@ agx_status agx_sww_frame_async(agx_handle h, double min_storable_height, int32_t
  * into the page-locked buffer, valid until the next agx_sww_frame_async,
  * agx_sww_bind or destroy. */
 agx_status agx_sww_frame_wait(agx_handle h, const float** vertex, const float** centroid);
+/* As agx_sww_frame_wait, but the page-locked buffer itself (3P node values,
+ * then 3N centroid values) becomes the caller's until agx_frame_give: the
+ * frame is read where the device wrote it.  AGX_E_NOMEM when the callers
+ * together hold 1 GiB already (take the copy of agx_sww_frame_wait then).
+ * Thread safe; the buffer outlives the scenario. */
+agx_status agx_sww_frame_take(agx_handle h, float** frame);
+void agx_frame_give(float* frame);
 
 /* ---- diagnostics ------------------------------------------------------------- */
 int32_t agx_last_error(char* buf, int32_t n);
