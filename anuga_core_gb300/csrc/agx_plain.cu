@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(XTPB, AGX_MINB_EXTRAP) k_extrap(Dev d) {
     const double beta1 = q < 2 ? P.beta_w1 : q == 2 ? P.beta_uh1 : P.beta_vh1;
     const double inv1 = q < 2 ? P.inv_beta_w1 : q == 2 ? P.inv_beta_uh1 : P.inv_beta_vh1;
     const double beta = one ? beta1 : beta0_dry + (beta0 - beta0_dry) * f;
-    if (dgt0(beta)) limited_edges(qc, jump, limiter_phi(jump, lo, hi, beta, one ? inv1 : 0.0), E);
+    if (dgt0(beta)) limited_edges<IM>(qc, jump, limiter_phi<IM>(jump, lo, hi, beta, one ? inv1 : 0.0), E);
   } else if (nb == 2) {
     const double qn = s.x != k ? q0 : (s.y != k ? q1 : q2);
     reconstruct_towards(P.beta_w, P.inv_beta_w, qc, qn, G, E);
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(XTPB, AGX_MINB_EXTRAP) k_extrap(Dev d) {
   const size_t b = 3 * (size_t)k;
   if (q >= 2 && P.velocity_extrapolation) {
 #pragma unroll
-    for (int i = 0; i < 3; i++) E[i] = E[i] * s_h[i][lane];
+    for (int i = 0; i < 3; i++) E[i] = imul<IM>(E[i], s_h[i][lane]);
   }
   double* const out = q == 0 ? d.we : q == 1 ? d.he : q == 2 ? d.uhe : d.vhe;
 #pragma unroll

@@ -263,6 +263,7 @@ AGX_HD double min_failing_ratio(const bool fail[3], const bool neg[3], double lo
 }
 
 // inv_known > 0 is 1/beta, formed beforehand; otherwise it is divided out.
+template <bool IM = false>
 AGX_HD double limiter_phi(const double jump[3], double lo, double hi, double beta, double inv_known) {
   const double tiny = 1.0e-100;
   // The reference's phi = fmin(fmin(floor, r_0, r_1, r_2) * beta, 1) over the
@@ -293,12 +294,13 @@ AGX_HD double limiter_phi(const double jump[3], double lo, double hi, double bet
     return dmin(min_failing_ratio(fail, neg, lo, hi, jump, ratio_floor), 1.0);
   }
   if (dgt0(beta)) {
-    const double inv_beta = dgt0(inv_known) ? inv_known : 1.0 / beta;
+    const double inv_beta = dgt0(inv_known) ? inv_known : ddiv(1.0, beta);
     const double need = inv_beta * (1.0 + 9.094947017729282e-13);
     bool fail[3], any = false;
     for (int i = 0; i < 3; i++) {
       // ratio lo/d with both negative: lo/d >= need  <=>  lo <= d*need
-      fail[i] = neg[i] ? !dle(lo, jump[i] * need) : (pos[i] && !dge(hi, jump[i] * need));
+      const double jn = imul<IM>(jump[i], need);
+      fail[i] = neg[i] ? !dle(lo, jn) : (pos[i] && !dge(hi, jn));
       any |= fail[i];
     }
     if (!any && dle(inv_beta, ratio_floor)) return dmin(ratio_floor * beta, 1.0);
@@ -320,13 +322,20 @@ AGX_HD double limiter_phi(const double jump[3], double lo, double hi, double bet
 //   nb==2 : g[6]=gradient factor x, g[7]=gradient factor y
 constexpr int GEO_STRIDE = 11;
 
-// Edge values qc + jump * phi (jump * 1 is jump: the product is skipped).
+// Edge values qc + jump * phi.  Only limited cells take the products (jump * 1
+// is jump); the sums stand after them, so that the limited and the other
+// lanes of a warp share them.
+template <bool IM = false>
 AGX_HD void limited_edges(double qc, const double jump[3], double phi, double out[3]) {
-  if (dbits(phi) == dbits(1.0)) {
-    for (int i = 0; i < 3; i++) out[i] = qc + jump[i];
-  } else {
-    for (int i = 0; i < 3; i++) out[i] = qc + jump[i] * phi;
+  double j0 = jump[0], j1 = jump[1], j2 = jump[2];
+  if (dbits(phi) != dbits(1.0)) {
+    j0 = imul<IM>(j0, phi);
+    j1 = imul<IM>(j1, phi);
+    j2 = imul<IM>(j2, phi);
   }
+  out[0] = qc + j0;
+  out[1] = qc + j1;
+  out[2] = qc + j2;
 }
 
 // The jumps to the three edges (the auxiliary triangle's gradient over the
