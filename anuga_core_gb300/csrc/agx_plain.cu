@@ -23,18 +23,18 @@ namespace agx {
 // blocks of a mesh of some tens of thousands of cells spread evenly over the
 // 152 SMs (40,000 cells: 157 blocks of 256 gave five SMs twice the work).
 constexpr int TPB = 128;
-// resident blocks of 128 per SM asked of the compiler (register budgets): 64
-// registers for the extrapolation, the flux and the update, and for the
-// accumulation on large meshes (8577 against 8616 us a 4.0M-triangle run with
-// 80, 10 blocks of the extrapolation 8590, 6 of the flux 8645)
+// resident blocks of 128 per SM asked of the compiler (register budgets),
+// measured on the 4.0M-triangle DE1 run: extrapolation 8 (6: +2%, 10: the
+// same and +4% at 40,000 cells), flux 7 (8: +0.5%), update 10 (8: +1%, 12: the
+// same), accumulation 8 on large meshes (5: +0.5%)
 #ifndef AGX_MINB_EXTRAP
 #define AGX_MINB_EXTRAP 8
 #endif
 #ifndef AGX_MINB_FLUX
-#define AGX_MINB_FLUX 8
+#define AGX_MINB_FLUX 7
 #endif
 #ifndef AGX_MINB_UPDATE
-#define AGX_MINB_UPDATE 8
+#define AGX_MINB_UPDATE 10
 #endif
 
 __device__ __forceinline__ double warp_sum(double x) {
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(XTPB, AGX_MINB_EXTRAP) k_extrap(Dev d) {
     const double beta1 = q < 2 ? P.beta_w1 : q == 2 ? P.beta_uh1 : P.beta_vh1;
     const double inv1 = q < 2 ? P.inv_beta_w1 : q == 2 ? P.inv_beta_uh1 : P.inv_beta_vh1;
     const double beta = one ? beta1 : beta0_dry + (beta0 - beta0_dry) * f;
-    if (dgt0(beta)) limited_edges<IM>(qc, jump, limiter_phi<IM>(jump, lo, hi, beta, one ? inv1 : 0.0), E);
+    if (dgt0(beta)) limited_edges(qc, jump, limiter_phi(jump, lo, hi, beta, one ? inv1 : 0.0), E);
   } else if (nb == 2) {
     const double qn = s.x != k ? q0 : (s.y != k ? q1 : q2);
     reconstruct_towards(P.beta_w, P.inv_beta_w, qc, qn, G, E);
@@ -669,8 +669,10 @@ __global__ void k_clock(Dev d, cudaGraphConditionalHandle handle, int set_cond) 
 
 // ---------------------------------------------------------------------------
 static inline int nblk(int n) { return (n + TPB - 1) / TPB; }
-// Meshes from here on take the integer products (see imul).
-constexpr int IMUL_MIN_CELLS = 60000;
+// Meshes from here on take the integer products (see imul): 40,000 cells 2772
+// us a run with them and 2922 without, 396 cells the other way round; at
+// 20,000 cells a block of four warps per SM is all there is.
+constexpr int IMUL_MIN_CELLS = 20000;
 static inline int xblk(int n) { return (n + XCELLS - 1) / XCELLS; }
 
 #define LAUNCHK(cat, ...)                  \

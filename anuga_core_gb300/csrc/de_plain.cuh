@@ -110,15 +110,16 @@ AGX_HD double dsqrt(double x) {
 }
 
 // A product formed with integer instructions on the device (the same bits)
-// where ON.  The extrapolation and the flux keep the FP64 pipe 76-78% busy
-// and the issue slots 16-28% on a large mesh: products moved to the integer
-// pipes run beside it until the two balance.  Per 4.0M-triangle DE1 step,
-// from 4.58 ms with none: 4.31 with the gradients' four products a quantity, the
-// eight rotations of an edge's momenta and the accumulation's normals, 4.15
-// with eight a quantity, 4.04 with 25 an edge as well (twelve a quantity 4.17:
-// past the balance; the accumulation's other products nothing on 250,000).
-// On a small mesh nothing fills the pipes and an integer product only takes
-// longer (396 cells: 840 against 974 us a run), so the kernels take a switch.
+// where ON.  With FP64 products alone the extrapolation and the flux kept the
+// FP64 pipe 76-78% busy and the issue slots 16-28% on a large mesh: products
+// moved to the integer pipes run beside it until neither is the limit.  Per
+// 4.0M-triangle DE1 step, from 4.58 ms with none: 4.31 with the gradients'
+// four products a quantity, the eight rotations of an edge's momenta and the
+// accumulation's normals, 4.15 with eight a quantity, 4.04 with 25 an edge as
+// well; twelve a quantity or the limiter's products too are past the balance
+// (+1 to +3%), the accumulation's others cost 3% on 250,000 cells.  On a small
+// mesh nothing fills the pipes and an integer product only takes longer, so
+// the kernels take a switch.
 template <bool ON>
 AGX_HD double imul(double a, double b) {
 #if defined(__CUDA_ARCH__)
@@ -263,7 +264,6 @@ AGX_HD double min_failing_ratio(const bool fail[3], const bool neg[3], double lo
 }
 
 // inv_known > 0 is 1/beta, formed beforehand; otherwise it is divided out.
-template <bool IM = false>
 AGX_HD double limiter_phi(const double jump[3], double lo, double hi, double beta, double inv_known) {
   const double tiny = 1.0e-100;
   // The reference's phi = fmin(fmin(floor, r_0, r_1, r_2) * beta, 1) over the
@@ -299,7 +299,7 @@ AGX_HD double limiter_phi(const double jump[3], double lo, double hi, double bet
     bool fail[3], any = false;
     for (int i = 0; i < 3; i++) {
       // ratio lo/d with both negative: lo/d >= need  <=>  lo <= d*need
-      const double jn = imul<IM>(jump[i], need);
+      const double jn = jump[i] * need;
       fail[i] = neg[i] ? !dle(lo, jn) : (pos[i] && !dge(hi, jn));
       any |= fail[i];
     }
@@ -325,13 +325,12 @@ constexpr int GEO_STRIDE = 11;
 // Edge values qc + jump * phi.  Only limited cells take the products (jump * 1
 // is jump); the sums stand after them, so that the limited and the other
 // lanes of a warp share them.
-template <bool IM = false>
 AGX_HD void limited_edges(double qc, const double jump[3], double phi, double out[3]) {
   double j0 = jump[0], j1 = jump[1], j2 = jump[2];
   if (dbits(phi) != dbits(1.0)) {
-    j0 = imul<IM>(j0, phi);
-    j1 = imul<IM>(j1, phi);
-    j2 = imul<IM>(j2, phi);
+    j0 = j0 * phi;
+    j1 = j1 * phi;
+    j2 = j2 * phi;
   }
   out[0] = qc + j0;
   out[1] = qc + j1;

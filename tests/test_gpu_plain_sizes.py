@@ -1,6 +1,6 @@
 """Plain FP64 step kernels at the sizes where their blocks end and their
 dispatch changes: meshes of 4 to a few hundred triangles around the kernels'
-32- and 128-cell blocks, and of 59,400 and 61,004, three steps of each flow algorithm without friction, bit for bit the
+32- and 128-cell blocks, and of 19,800 and 20,200, three steps of each flow algorithm without friction, bit for bit the
 oracle's (no tolerance: the FP64 form rounds every operation as the oracle
 does)."""
 import numpy as np
@@ -13,9 +13,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("alg", ["DE0", "DE1", "DE2", "DE0_7"])
-# the last two sit on both sides of the 60,000 cells from which the kernels form products with integer instructions
+# the last two sit on both sides of the 20,000 cells from which the kernels form products with integer instructions
 @pytest.mark.parametrize("m,n", [(1, 1), (7, 1), (8, 1), (9, 1), (4, 4), (17, 1), (8, 4), (3, 11), (16, 16), (13, 21),
-                                 (150, 99), (151, 101)])
+                                 (99, 50), (101, 50)])
 def test_steps_bitwise_at_block_ends(oracle_mod, alg, m, n):
     p, e, b = rectangular_cross(m, n, 10.0 * m, 10.0 * n)
     mesh = Mesh(p, e, b)
