@@ -78,15 +78,6 @@ SF_HD int clz64(uint64_t x) {
 #endif
 }
 
-// the high 64 bits of the 128-bit product a * b
-SF_HD uint64_t mulhi64(uint64_t a, uint64_t b) {
-#ifdef __CUDA_ARCH__
-  return __umul64hi(a, b);
-#else
-  return (uint64_t)(((unsigned __int128)a * b) >> 64);
-#endif
-}
-
 // x >> n with every bit shifted out ORed into bit 0 (n >= 0)
 SF_HD uint64_t shr_jam(uint64_t x, int n) {
   if (n <= 0) return x;

@@ -438,15 +438,15 @@ def measure_single(args, precision, torch, world, barrier, dist, builder):
 # FP64-pipe instructions per cell of one DE1 step (two stages) of the plain
 # path, from one ncu capture (sm__thread_inst_executed_pipe_fp64_pred_on.sum:
 # lanes that did work; sm__inst_executed_pipe_fp64.sum x 32: lane slots the
-# warps occupied, idle lanes of divergent branches included) of each kernel
-# of a stage (prep, extrapolation, flux, accumulation, update) on the
-# 1.0M-triangle inflow_bumps case, divided by its cells, times two stages.
+# warps occupied, idle lanes of divergent branches included) of every kernel
+# of the step (prep, then extrapolation, flux, accumulation and update of both
+# stages) on the 1.0M-triangle inflow_bumps case, divided by its cells.
 FP64_PER_CELL_STEP = {
-    "lane_ops": 2 * (7.241 + 102.7 + 102.9 + 55.64 + 52.47),
-    "warp_slots": 2 * 32 * (2.318e5 + 3.958e6 + 3.516e6 + 1.820e6 + 1.690e6) / 1.0e6,
+    "lane_ops": 3.395 + (72.78 + 58.57 + 36.01 + 27.91) + (72.78 + 58.58 + 35.02 + 26.96),
+    "warp_slots": 3.469 + (77.01 + 70.57 + 37.84 + 28.75) + (77.01 + 70.57 + 36.63 + 30.67),
     "note": "ncu --metrics sm__thread_inst_executed_pipe_fp64_pred_on.sum,sm__inst_executed_pipe_fp64.sum of "
-            "k_prep, k_extrap<0,1>, k_flux, k_accum, k_update on the 1.0M-triangle inflow_bumps case (m=500), "
-            "per cell and launch, x 2 stages of a DE1 step"}
+            "k_prep, k_extrap<0,1>, k_flux<1,1>, k_accum<1>, k_update<1> and <0> on the 1.0M-triangle inflow_bumps "
+            "case (m=500), per cell, over the launches of one DE1 step"}
 
 
 def fp64_roofline(cells, ms_per_step, dfma_gops):
@@ -465,15 +465,17 @@ def fp64_roofline(cells, ms_per_step, dfma_gops):
 
 TRAFFIC_PER_STEP = {
     ("mixed", "flux"): {
-        "bytes_per_cell": (117.678592e6 + 15.682304e6 + 177.783552e6 + 32.170752e6) / 1.0e6,
+        "bytes_per_cell": (117.650432e6 + 14.409472e6 + 177.769216e6 + 33.533184e6) / 1.0e6,
         "note": "ncu --set full of k_pool_flux stage 1 + stage 2 on the 1.0M-triangle inflow_bumps case "
                 "(m=500, MINB=8 variant), dram__bytes_read.sum + dram__bytes_write.sum per step, "
                 "scaled by cells"},
     ("fp64", "extrap"): {
-        "bytes_per_cell": 2 * (137.848576e6 + 85.762944e6) / 1.0e6,
-        "note": "ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum of k_extrap<0,1> (edges only, cells in "
-                "branch-class order, flowing state) on the 1.0M-triangle inflow_bumps case (m=500), per launch x 2 "
-                "launches per DE1 step, scaled by cells"},
+        "bytes_per_cell": (126.836e6 + 84.865e6 + 126.866e6 + 84.921e6) / 1.0e6,
+        "note": "ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum of k_extrap<0,1> (edges only, flowing "
+                "state) on the 1.0M-triangle inflow_bumps case (m=500), both launches of a DE1 step, scaled by cells"},
+    ("fp64", "flux"): {
+        "bytes_per_cell": (240.537e6 + 106.451e6 + 240.603e6 + 106.222e6) / 1.0e6,
+        "note": "the same of k_flux<1,1>"},
 }
 
 
