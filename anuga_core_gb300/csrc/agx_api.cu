@@ -1,13 +1,12 @@
 // agx_api.cu -- C ABI of libagx: scenario lifetime, state access, per-phase
 // calls and the graph-captured device step loop.
 #include "agx_internal.cuh"
+#include "frame_buffers.h"
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
-#include <unordered_map>
-#include <unordered_set>
 
 namespace agx {
 
@@ -79,85 +78,26 @@ static agx_status fail(agx_status code, const char* fmt, ...) {
   } while (0)
 
 // ---- output frame buffers ------------------------------------------------
-namespace {
-struct FrameBuffers {
-  std::mutex mu;
-  std::unordered_map<float*, size_t> size;              // every live buffer
-  std::unordered_multimap<size_t, float*> kept;
-  std::unordered_set<float*> taken;
-  size_t kept_bytes = 0, taken_bytes = 0;
-};
+static float* page_locked(size_t bytes) {
+  float* p = nullptr;
+  if (cudaMallocHost(&p, bytes) == cudaSuccess) return p;
+  cudaGetLastError();                    // the caller reports it
+  return nullptr;
+}
+static void page_unlocked(float* p) { cudaFreeHost(p); }
 // never destroyed: arrays that hold a frame may outlive the library's statics
-FrameBuffers& frame_buffers() {
-  static FrameBuffers* b = new FrameBuffers();
+static FrameBuffers& frame_buffers() {
+  static FrameBuffers* b = new FrameBuffers(page_locked, page_unlocked);
   return *b;
 }
-}  // namespace
 
 cudaError_t frame_buffer_get(size_t bytes, float** out) {
-  FrameBuffers& B = frame_buffers();
-  {
-    std::lock_guard<std::mutex> lock(B.mu);
-    auto it = B.kept.find(bytes);
-    if (it != B.kept.end()) {
-      *out = it->second;
-      B.kept.erase(it);
-      B.kept_bytes -= bytes;
-      return cudaSuccess;
-    }
-  }
-  float* p = nullptr;
-  const cudaError_t e = cudaMallocHost(&p, bytes);
-  if (e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> lock(B.mu);
-  B.size[p] = bytes;
-  *out = p;
-  return cudaSuccess;
+  *out = frame_buffers().get(bytes);
+  return *out ? cudaSuccess : cudaErrorMemoryAllocation;
 }
-
-bool frame_buffer_take(float* p) {
-  FrameBuffers& B = frame_buffers();
-  std::lock_guard<std::mutex> lock(B.mu);
-  const size_t bytes = B.size[p];
-  if (B.taken_bytes + bytes > FRAME_TAKEN) return false;
-  B.taken.insert(p);
-  B.taken_bytes += bytes;
-  return true;
-}
-
-void frame_buffer_give(float* p) {
-  FrameBuffers& B = frame_buffers();
-  {
-    std::lock_guard<std::mutex> lock(B.mu);
-    auto it = B.size.find(p);
-    if (it == B.size.end()) return;
-    const size_t bytes = it->second;
-    if (B.taken.erase(p)) B.taken_bytes -= bytes;
-    if (B.kept_bytes + bytes <= FRAME_KEEP) {
-      B.kept.emplace(bytes, p);
-      B.kept_bytes += bytes;
-      return;
-    }
-    B.size.erase(it);
-  }
-  cudaFreeHost(p);
-}
-
-void frame_buffer_release(float* p, size_t bytes) {
-  FrameBuffers& B = frame_buffers();
-  std::vector<float*> gone;
-  {
-    std::lock_guard<std::mutex> lock(B.mu);
-    if (p && B.size.erase(p)) gone.push_back(p);
-    for (auto it = B.kept.find(bytes); it != B.kept.end(); it = B.kept.find(bytes)) {
-      gone.push_back(it->second);
-      B.size.erase(it->second);
-      B.kept.erase(it);
-      B.kept_bytes -= bytes;
-    }
-  }
-  for (float* q : gone) cudaFreeHost(q);
-}
+bool frame_buffer_take(float* p) { return frame_buffers().take(p); }
+void frame_buffer_give(float* p) { frame_buffers().give(p); }
+void frame_buffer_release(float* p, size_t bytes) { frame_buffers().release(p, bytes); }
 
 static size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 

@@ -249,17 +249,11 @@ struct TraceRange {
 };
 #define AGX_TRACE(name) ::agx::TraceRange agx_trace_range_(name)
 
-// Page-locked buffers of output frames (agx_api.cu).  A buffer belongs to a
-// scenario or, once taken, to a caller; one given back is kept for the next
-// frame of its size (page-locking 72 MB takes some 20 ms), at most
-// FRAME_KEEP bytes in all, and those of a size are released with a scenario
-// of that size.
-constexpr size_t FRAME_KEEP = 256u << 20;
-constexpr size_t FRAME_TAKEN = 1u << 30;     // bytes callers may hold
+// The process's page-locked buffers of output frames (frame_buffers.h).
 cudaError_t frame_buffer_get(size_t bytes, float** out);
-bool frame_buffer_take(float* p);            // false: the callers hold FRAME_TAKEN already
+bool frame_buffer_take(float* p);
 void frame_buffer_give(float* p);
-void frame_buffer_release(float* p, size_t bytes);   // p (may be null) and the kept ones of its size
+void frame_buffer_release(float* p, size_t bytes);
 
 // launch accounting
 void count_launch(int64_t n = 1);

@@ -280,6 +280,8 @@ agx_status agx_sww_frame_wait(agx_handle h, const float** vertex, const float** 
  * together hold 1 GiB already (take the copy of agx_sww_frame_wait then).
  * Thread safe; the buffer outlives the scenario. */
 agx_status agx_sww_frame_take(agx_handle h, float** frame);
+/* Gives a taken buffer back; a pointer that is not a caller's (given back
+ * already, or a scenario's own) is ignored. */
 void agx_frame_give(float* frame);
 
 /* ---- diagnostics ------------------------------------------------------------- */
