@@ -91,13 +91,17 @@ static FrameBuffers& frame_buffers() {
   return *b;
 }
 
+cudaError_t frame_buffer_enter(size_t bytes, float** out) {
+  *out = frame_buffers().enter(bytes);
+  return *out ? cudaSuccess : cudaErrorMemoryAllocation;
+}
+void frame_buffer_leave(float* p, size_t bytes) { frame_buffers().leave(p, bytes); }
 cudaError_t frame_buffer_get(size_t bytes, float** out) {
   *out = frame_buffers().get(bytes);
   return *out ? cudaSuccess : cudaErrorMemoryAllocation;
 }
 bool frame_buffer_take(float* p) { return frame_buffers().take(p); }
 void frame_buffer_give(float* p) { frame_buffers().give(p); }
-void frame_buffer_release(float* p, size_t bytes) { frame_buffers().release(p, bytes); }
 
 static size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -361,10 +365,8 @@ agx_status agx_scenario_destroy(agx_handle h) {
     cudaStreamSynchronize(s->copy_stream);
     cudaStreamDestroy(s->copy_stream);
   }
-  if (s->frame) {
-    cudaFree(s->frame);
-    frame_buffer_release(s->frame_host, s->frame_bytes);
-  }
+  if (s->frame) cudaFree(s->frame);
+  if (s->frame_bytes) frame_buffer_leave(s->frame_host, s->frame_bytes);
   if (s->frame_done) cudaEventDestroy(s->frame_done);
   if (s->frame_ready) cudaEventDestroy(s->frame_ready);
   if (s->bseries) cudaFree(s->bseries);
@@ -431,10 +433,9 @@ agx_status agx_sww_bind(agx_handle h, int64_t P, const int32_t* node_offsets, co
   if (h->node_off) cudaFree(h->node_off);
   if (h->node_slot) cudaFree(h->node_slot);
   if (h->copy_stream) CK(cudaStreamSynchronize(h->copy_stream));
-  if (h->frame) {
-    cudaFree(h->frame);
-    frame_buffer_release(h->frame_host, h->frame_bytes);
-  }
+  if (h->frame) cudaFree(h->frame);
+  if (h->frame_bytes) frame_buffer_leave(h->frame_host, h->frame_bytes);
+  h->frame_bytes = 0;
   if (h->frame_done) cudaEventDestroy(h->frame_done);
   if (h->frame_ready) cudaEventDestroy(h->frame_ready);
   h->node_off = h->node_slot = nullptr;
@@ -445,8 +446,8 @@ agx_status agx_sww_bind(agx_handle h, int64_t P, const int32_t* node_offsets, co
   CK(cudaMalloc(&h->node_off, (size_t)(P + 1) * 4));
   CK(cudaMalloc(&h->node_slot, (size_t)3 * h->N * 4 + 4));
   CK(cudaMalloc(&h->frame, fbytes));
+  CK(frame_buffer_enter(fbytes, &h->frame_host));
   h->frame_bytes = fbytes;
-  CK(frame_buffer_get(fbytes, &h->frame_host));
   CK(cudaEventCreateWithFlags(&h->frame_done, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&h->frame_ready, cudaEventDisableTiming));
   if (!h->copy_stream) CK(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));

@@ -212,7 +212,7 @@ struct Scenario {
   int* node_slot = nullptr;
   float* frame = nullptr;
   float* frame_host = nullptr;           // page-locked copy of the last frame (null once taken)
-  size_t frame_bytes = 0;
+  size_t frame_bytes = 0;                // of that copy; 0: not bound for output
   cudaEvent_t frame_done = nullptr;      // recorded after that copy
   cudaEvent_t frame_ready = nullptr;     // recorded after the frame kernels
   cudaStream_t copy_stream = nullptr;    // the copy's own stream: the next steps need not wait for it
@@ -250,10 +250,11 @@ struct TraceRange {
 #define AGX_TRACE(name) ::agx::TraceRange agx_trace_range_(name)
 
 // The process's page-locked buffers of output frames (frame_buffers.h).
+cudaError_t frame_buffer_enter(size_t bytes, float** out);
+void frame_buffer_leave(float* p, size_t bytes);
 cudaError_t frame_buffer_get(size_t bytes, float** out);
 bool frame_buffer_take(float* p);
 void frame_buffer_give(float* p);
-void frame_buffer_release(float* p, size_t bytes);
 
 // launch accounting
 void count_launch(int64_t n = 1);

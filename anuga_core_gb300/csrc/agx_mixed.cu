@@ -1483,10 +1483,9 @@ static void free_sww(ScnHost& s) {
   }
   if (s.sww_off) cudaFree(s.sww_off);
   if (s.sww_slot) cudaFree(s.sww_slot);
-  if (s.frame) {
-    cudaFree(s.frame);
-    frame_buffer_release(s.frame_host, s.frame_bytes);
-  }
+  if (s.frame) cudaFree(s.frame);
+  if (s.frame_bytes) frame_buffer_leave(s.frame_host, s.frame_bytes);
+  s.frame_bytes = 0;
   if (s.frame_done) cudaEventDestroy(s.frame_done);
   if (s.frame_ready) cudaEventDestroy(s.frame_ready);
   s.sww_off = s.sww_slot = nullptr;
@@ -2657,8 +2656,8 @@ agx_status agx_pool_sww_bind(agx_pool p, int32_t sid, int64_t P, const int32_t* 
   PCK(cudaMalloc(&sh.sww_off, (size_t)(P + 1) * 4));
   PCK(cudaMalloc(&sh.sww_slot, (size_t)S3 * 4 + 4));
   PCK(cudaMalloc(&sh.frame, fbytes));
+  PCK(frame_buffer_enter(fbytes, &sh.frame_host));
   sh.frame_bytes = fbytes;
-  PCK(frame_buffer_get(fbytes, &sh.frame_host));
   PCK(cudaEventCreateWithFlags(&sh.frame_done, cudaEventDisableTiming));
   PCK(cudaEventCreateWithFlags(&sh.frame_ready, cudaEventDisableTiming));
   PCK(cudaStreamCreateWithFlags(&sh.copy_stream, cudaStreamNonBlocking));

@@ -1,7 +1,8 @@
 """Ownership of the output frames' page-locked buffers (anuga_core_gb300/csrc/
 frame_buffers.h, compiled by g++ on the host with the heap in their place;
 tests/cpp/check_frame_buffers.cpp): no buffer has two owners, whatever callers
-give back."""
+give back, no steady loop page-locks memory, and what is page-locked stays
+bounded."""
 import os
 import shutil
 import subprocess
