@@ -503,7 +503,7 @@ agx_status agx_sww_frame_take(agx_handle h, float** frame) {
   if (!h->frame) return fail(AGX_E_STATE, "agx_sww_bind first");
   agx_status st = frame_on_host(h);
   if (st) return st;
-  if (!frame_buffer_take(h->frame_host)) return fail(AGX_E_NOMEM, "callers hold 1 GiB of frames");
+  if (!frame_buffer_take(h->frame_host)) return fail(AGX_E_NOMEM, "callers hold 1 GiB of frames, or this one is not page-locked");
   *frame = h->frame_host;
   h->frame_host = nullptr;
   return AGX_OK;

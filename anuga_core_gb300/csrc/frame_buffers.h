@@ -2,6 +2,7 @@
 // (plain C++, so that it is checked on the host with other allocators).
 #pragma once
 #include <cstddef>
+#include <cstdlib>
 #include <list>
 #include <mutex>
 #include <unordered_map>
@@ -11,12 +12,16 @@ namespace agx {
 // Each scenario that is bound for output has one buffer.  A caller may take it
 // as it is (TAKEN bytes in all, beyond that callers copy); the scenario's next
 // frame then needs another, and one given back is kept for that (288 MB: 2.9
-// ms a frame, 12.7 with a buffer page-locked for each, 27 copied).  Kept are, of each size, as many as its
-// scenarios are without and two a scenario beyond those (a caller that
-// replaces its last frame by the next holds two), KEEP bytes of the latter in
-// all, the oldest going first; of a size no scenario has any more, none.  A
-// loop that takes and gives back within these bounds neither page-locks nor
-// frees.  Safe from several threads.
+// ms a frame, 12.7 with a buffer page-locked for each, 27 copied).  Kept are,
+// of each size, as many as its scenarios are without and two a scenario beyond
+// those (a caller that replaces its last frame by the next holds two), KEEP
+// bytes of the latter in all, the oldest going first; of a size no scenario
+// has any more, none.  A loop that takes and gives back within these bounds
+// neither page-locks nor frees.
+// Where no more memory can be page-locked the kept buffers are released; a
+// scenario that still gets none has its frames in pageable memory (slower to
+// copy to, never a caller's), so a run that could be bound does not fail later.
+// Safe from several threads.
 class FrameBuffers {
  public:
   static constexpr size_t KEEP = 1u << 30;
@@ -31,7 +36,7 @@ class FrameBuffers {
       std::lock_guard<std::mutex> lock(mu_);
       sizes_[bytes].bound++;
     }
-    float* p = get(bytes);
+    float* p = get(bytes, true);
     if (!p) leave(nullptr, bytes);
     return p;
   }
@@ -45,17 +50,23 @@ class FrameBuffers {
       z.bound--;
       if (p) {
         z.owned--;
-        keep(p, bytes);
+        const auto it = live_.find(p);
+        if (it->second.pageable) {
+          live_.erase(it);
+          std::free(p);
+        } else {
+          keep(p, bytes);
+        }
       }
       trim(bytes, gone);
     }
     for (const Kept& k : gone) free_(k.p);
   }
 
-  // a buffer for a scenario whose last one was taken, or null
-  float* get(size_t bytes) {
+  // a buffer for a scenario whose last one was taken; `lock`: page-locked or null
+  float* get(size_t bytes, bool lock = false) {
     {
-      std::lock_guard<std::mutex> lock(mu_);
+      std::lock_guard<std::mutex> guard(mu_);
       Size& z = sizes_[bytes];
       z.owned++;
       if (z.kept > 0) {
@@ -69,17 +80,24 @@ class FrameBuffers {
       }
     }
     float* p = alloc_(bytes);
-    std::lock_guard<std::mutex> lock(mu_);
-    if (p) live_[p] = {bytes, false};
+    if (!p) {
+      release_kept();
+      p = alloc_(bytes);
+    }
+    const bool pageable = !p && !lock;
+    if (pageable) p = (float*)std::malloc(bytes);
+    std::lock_guard<std::mutex> guard(mu_);
+    if (p) live_[p] = {bytes, false, pageable};
     else sizes_[bytes].owned--;
     return p;
   }
 
-  // a scenario's buffer becomes the caller's; false: the callers hold TAKEN already
+  // a scenario's buffer becomes the caller's; false: the callers hold TAKEN
+  // already, or it is not page-locked
   bool take(float* p) {
     std::lock_guard<std::mutex> lock(mu_);
     const auto it = live_.find(p);
-    if (it == live_.end() || it->second.taken) return false;
+    if (it == live_.end() || it->second.taken || it->second.pageable) return false;
     const size_t bytes = it->second.bytes;
     if (taken_bytes_ + bytes > TAKEN) return false;
     it->second.taken = true;
@@ -114,7 +132,7 @@ class FrameBuffers {
   };
   struct Live {
     size_t bytes;
-    bool taken;
+    bool taken, pageable;
   };
   struct Kept {
     float* p;
@@ -130,6 +148,15 @@ class FrameBuffers {
     live_.erase(it->p);
     sizes_[it->bytes].kept--;
     gone.splice(gone.end(), kept_, it);
+  }
+
+  void release_kept() {
+    std::list<Kept> gone;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      while (!kept_.empty()) drop(kept_.begin(), gone);
+    }
+    for (const Kept& k : gone) free_(k.p);
   }
 
   // kept buffers beyond the bounds go: of this size, then the oldest of any

@@ -277,7 +277,8 @@ agx_status agx_sww_frame_wait(agx_handle h, const float** vertex, const float** 
 /* As agx_sww_frame_wait, but the page-locked buffer itself (3P node values,
  * then 3N centroid values) becomes the caller's until agx_frame_give: the
  * frame is read where the device wrote it.  AGX_E_NOMEM when the callers
- * together hold 1 GiB already (take the copy of agx_sww_frame_wait then).
+ * together hold 1 GiB already or no memory could be page-locked for this frame
+ * (take the copy of agx_sww_frame_wait then).
  * Thread safe; the buffer outlives the scenario. */
 agx_status agx_sww_frame_take(agx_handle h, float** frame);
 /* Gives a taken buffer back; a pointer that is not a caller's (given back

@@ -6,6 +6,7 @@
 #include <cstdlib>
 #include <deque>
 #include <functional>
+#include <set>
 #include <thread>
 #include <vector>
 #include "../../anuga_core_gb300/csrc/frame_buffers.h"
@@ -13,6 +14,15 @@
 using agx::FrameBuffers;
 
 constexpr size_t MB = 1u << 20;
+
+static long g_bad = 0;
+#define EXPECT(cond)                                              \
+  do {                                                            \
+    if (!(cond)) {                                                \
+      std::printf("line %d: %s does not hold\n", __LINE__, #cond); \
+      g_bad++;                                                    \
+    }                                                             \
+  } while (0)
 
 static std::atomic<long> g_allocs{0}, g_frees{0};
 static float* heap_alloc(size_t bytes) {
@@ -23,15 +33,19 @@ static void heap_free(float* p) {
   g_frees++;
   std::free(p);
 }
-
-static long g_bad = 0;
-#define EXPECT(cond)                                              \
-  do {                                                            \
-    if (!(cond)) {                                                \
-      std::printf("line %d: %s does not hold\n", __LINE__, #cond); \
-      g_bad++;                                                    \
-    }                                                             \
-  } while (0)
+// the same where only `g_room` buffers can be page-locked
+static long g_room = 0;
+static std::set<float*> g_locked;
+static float* scarce_alloc(size_t bytes) {
+  if ((long)g_locked.size() >= g_room) return nullptr;
+  float* p = heap_alloc(bytes);
+  g_locked.insert(p);
+  return p;
+}
+static void scarce_free(float* p) {
+  EXPECT(g_locked.erase(p) == 1);
+  heap_free(p);
+}
 
 // A buffer given back twice, one a scenario still owns, and a pointer that is
 // no buffer: only a caller's buffer goes back.
@@ -193,6 +207,44 @@ static void check_room() {
   EXPECT(live() == before);
 }
 
+// No more memory can be page-locked: kept buffers make room, then frames go
+// through pageable memory and are not handed over; a scenario that cannot be
+// bound says so.
+static void check_scarce() {
+  FrameBuffers B(scarce_alloc, scarce_free);
+  g_room = 3;
+  {
+    Scenario a(B, 4000);
+    EXPECT(a.own != nullptr);
+    float* p = a.frame();
+    float* q = (a.own = B.get(a.bytes), a.frame());
+    a.own = B.get(a.bytes);
+    EXPECT(p && q && a.own && p != q && g_locked.size() == 3);
+    B.give(q);                                    // kept: the next size may have its room
+    {
+      Scenario b(B, 8000);
+      EXPECT(b.own != nullptr && g_locked.size() == 3);
+      float* r = b.frame();
+      EXPECT(r != nullptr);
+      b.own = B.get(b.bytes);                     // all three are in use
+      EXPECT(b.own != nullptr && g_locked.count(b.own) == 0);
+      if (b.own) {
+        b.own[0] = 1.0f;
+        float* own = b.own;
+        EXPECT(b.frame() == nullptr && b.own == own);
+        B.give(own);                              // not a caller's
+        EXPECT(b.own[0] == 1.0f);
+      }
+      EXPECT(B.enter(8000) == nullptr);           // binding needs a page-locked one, as ever
+      B.give(r);
+      EXPECT(g_locked.size() == 3);
+    }
+    EXPECT(g_locked.size() == 2);
+    B.give(p);
+  }
+  EXPECT(g_locked.empty());
+}
+
 // Several threads, each with its own scenarios and frames: no buffer is in
 // two hands (each writes its mark over what it holds and finds it again).
 static void check_threads() {
@@ -234,6 +286,7 @@ int main() {
   check_callers(1, 1600 * MB, false);    // one frame beyond it: all are
   check_callers(3, 4000, true);
   check_room();
+  check_scarce();
   check_threads();
   std::printf("failures %ld\n", g_bad);
   return g_bad ? 1 : 0;
