@@ -456,11 +456,30 @@ agx_status agx_sww_bind(agx_handle h, int64_t P, const int32_t* node_offsets, co
   return sync(h);
 }
 
+// The last frame in the scenario's buffer; copied again from the device if
+// that buffer has been taken since.
+static agx_status frame_on_host(agx_handle h) {
+  if (!h->frame_host) {
+    CK(frame_buffer_get(h->frame_bytes, &h->frame_host));
+    CK(cudaMemcpyAsync(h->frame_host, h->frame, ((size_t)3 * h->P + 3 * (size_t)h->N) * 4, cudaMemcpyDeviceToHost,
+                       h->copy_stream));
+    CK(cudaEventRecord(h->frame_done, h->copy_stream));
+  }
+  CK(cudaEventSynchronize(h->frame_done));
+  return AGX_OK;
+}
+
 agx_status agx_sww_frame(agx_handle h, double min_storable_height, int32_t centroid_averaging, float* vertex_out,
                          float* centroid_out) {
   AGX_TRACE("agx_sww_frame");
   if (!h || !vertex_out || !centroid_out) return fail(AGX_E_INVALID, "bad arguments");
   if (!h->frame) return fail(AGX_E_STATE, "agx_sww_bind first");
+  // a taken frame can still be waited for again, which copies it from the
+  // device buffer that this one goes to
+  if (!h->frame_host && h->frame_bytes) {
+    agx_status st = frame_on_host(h);
+    if (st) return st;
+  }
   CK(cudaStreamWaitEvent(h->stream, h->frame_done, 0));     // an earlier asynchronous copy of the buffer
   CK(enqueue_sww_frame(h, h->stream, min_storable_height, centroid_averaging ? 1 : 0));
   if (h->P > 0) CK(cudaMemcpyAsync(vertex_out, h->frame, (size_t)3 * h->P * 4, cudaMemcpyDeviceToHost, h->stream));
@@ -482,19 +501,6 @@ agx_status agx_sww_frame_async(agx_handle h, double min_storable_height, int32_t
   CK(cudaMemcpyAsync(h->frame_host, h->frame, ((size_t)3 * h->P + 3 * (size_t)h->N) * 4, cudaMemcpyDeviceToHost,
                      h->copy_stream));
   CK(cudaEventRecord(h->frame_done, h->copy_stream));
-  return AGX_OK;
-}
-
-// The last frame in the scenario's buffer; copied again from the device if
-// that buffer has been taken since.
-static agx_status frame_on_host(agx_handle h) {
-  if (!h->frame_host) {
-    CK(frame_buffer_get(h->frame_bytes, &h->frame_host));
-    CK(cudaMemcpyAsync(h->frame_host, h->frame, ((size_t)3 * h->P + 3 * (size_t)h->N) * 4, cudaMemcpyDeviceToHost,
-                       h->copy_stream));
-    CK(cudaEventRecord(h->frame_done, h->copy_stream));
-  }
-  CK(cudaEventSynchronize(h->frame_done));
   return AGX_OK;
 }
 
