@@ -436,6 +436,7 @@ agx_status agx_sww_bind(agx_handle h, int64_t P, const int32_t* node_offsets, co
   if (h->frame) cudaFree(h->frame);
   if (h->frame_bytes) frame_buffer_leave(h->frame_host, h->frame_bytes);
   h->frame_bytes = 0;
+  h->frame_only = false;
   if (h->frame_done) cudaEventDestroy(h->frame_done);
   if (h->frame_ready) cudaEventDestroy(h->frame_ready);
   h->node_off = h->node_slot = nullptr;
@@ -456,8 +457,8 @@ agx_status agx_sww_bind(agx_handle h, int64_t P, const int32_t* node_offsets, co
   return sync(h);
 }
 
-// The last frame in the scenario's buffer; copied again from the device if
-// that buffer has been taken since.
+// The frame started last in the scenario's buffer; copied again from the device
+// if that buffer has been taken since.  Under frame_mu.
 static agx_status frame_on_host(agx_handle h) {
   if (!h->frame_host) {
     CK(frame_buffer_get(h->frame_bytes, &h->frame_host));
@@ -475,10 +476,15 @@ agx_status agx_sww_frame(agx_handle h, double min_storable_height, int32_t centr
   if (!h || !vertex_out || !centroid_out) return fail(AGX_E_INVALID, "bad arguments");
   if (!h->frame) return fail(AGX_E_STATE, "agx_sww_bind first");
   // a taken frame can still be waited for again, which copies it from the
-  // device buffer that this one goes to
-  if (!h->frame_host && h->frame_bytes) {
-    agx_status st = frame_on_host(h);
-    if (st) return st;
+  // device buffer that this one goes to: it comes to the host first, and from
+  // there it is not handed over any more
+  if (h->frame_bytes) {
+    std::lock_guard<std::mutex> lock(h->frame_mu);
+    if (!h->frame_host) {
+      agx_status st = frame_on_host(h);
+      if (st) return st;
+    }
+    h->frame_only = true;
   }
   CK(cudaStreamWaitEvent(h->stream, h->frame_done, 0));     // an earlier asynchronous copy of the buffer
   CK(enqueue_sww_frame(h, h->stream, min_storable_height, centroid_averaging ? 1 : 0));
@@ -493,6 +499,8 @@ agx_status agx_sww_frame_async(agx_handle h, double min_storable_height, int32_t
   if (!h->frame) return fail(AGX_E_STATE, "agx_sww_bind first");
   // the frame kernels wait for the previous frame's copy to leave the buffer;
   // the copy runs on its own stream, so the steps enqueued next overlap it
+  std::lock_guard<std::mutex> lock(h->frame_mu);
+  h->frame_only = false;
   if (!h->frame_host) CK(frame_buffer_get(h->frame_bytes, &h->frame_host));     // the last one was taken
   CK(cudaStreamWaitEvent(h->stream, h->frame_done, 0));
   CK(enqueue_sww_frame(h, h->stream, min_storable_height, centroid_averaging ? 1 : 0));
@@ -507,9 +515,11 @@ agx_status agx_sww_frame_async(agx_handle h, double min_storable_height, int32_t
 agx_status agx_sww_frame_take(agx_handle h, float** frame) {
   if (!h || !frame) return fail(AGX_E_INVALID, "bad arguments");
   if (!h->frame) return fail(AGX_E_STATE, "agx_sww_bind first");
+  std::lock_guard<std::mutex> lock(h->frame_mu);
   agx_status st = frame_on_host(h);
   if (st) return st;
-  if (!frame_buffer_take(h->frame_host)) return fail(AGX_E_NOMEM, "callers hold 1 GiB of frames, or this one is not page-locked");
+  if (h->frame_only || !frame_buffer_take(h->frame_host))
+    return fail(AGX_E_NOMEM, "callers hold 1 GiB of frames, or this one cannot be handed over");
   *frame = h->frame_host;
   h->frame_host = nullptr;
   return AGX_OK;
@@ -520,6 +530,7 @@ void agx_frame_give(float* frame) { frame_buffer_give(frame); }
 agx_status agx_sww_frame_wait(agx_handle h, const float** vertex, const float** centroid) {
   if (!h || !vertex || !centroid) return fail(AGX_E_INVALID, "bad arguments");
   if (!h->frame) return fail(AGX_E_STATE, "agx_sww_bind first");
+  std::lock_guard<std::mutex> lock(h->frame_mu);
   agx_status st = frame_on_host(h);
   if (st) return st;
   *vertex = h->frame_host;

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 #include <stdint.h>
+#include <mutex>
 #include <string>
 #include <vector>
 #include <cstring>
@@ -213,6 +214,8 @@ struct Scenario {
   float* frame = nullptr;
   float* frame_host = nullptr;           // page-locked copy of the last frame (null once taken)
   size_t frame_bytes = 0;                // of that copy; 0: not bound for output
+  bool frame_only = false;               // the device buffer has another frame: the copy stays the scenario's
+  std::mutex frame_mu;                   // a frame may be waited for by a thread of its own
   cudaEvent_t frame_done = nullptr;      // recorded after that copy
   cudaEvent_t frame_ready = nullptr;     // recorded after the frame kernels
   cudaStream_t copy_stream = nullptr;    // the copy's own stream: the next steps need not wait for it

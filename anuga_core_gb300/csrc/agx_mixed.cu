@@ -2714,7 +2714,7 @@ agx_status agx_pool_sww_frame_take(agx_pool p, int32_t sid, float** frame) {
   if (!sh.frame) return pfail(AGX_E_STATE, "agx_pool_sww_bind first");
   agx_status st = frame_on_host(sh);
   if (st) return st;
-  if (!frame_buffer_take(sh.frame_host)) return pfail(AGX_E_NOMEM, "callers hold 1 GiB of frames, or this one is not page-locked");
+  if (!frame_buffer_take(sh.frame_host)) return pfail(AGX_E_NOMEM, "callers hold 1 GiB of frames, or this one cannot be handed over");
   *frame = sh.frame_host;
   sh.frame_host = nullptr;
   return AGX_OK;
