@@ -272,17 +272,21 @@ agx_status agx_sww_frame(agx_handle h, double min_storable_height, int32_t centr
 agx_status agx_sww_frame_async(agx_handle h, double min_storable_height, int32_t centroid_averaging);
 /* Wait for the frame started last; *vertex [3P] and *centroid [3N] point
  * into the page-locked buffer, valid until the next agx_sww_frame_async,
- * agx_sww_bind or destroy. */
+ * agx_sww_bind or destroy, or until agx_sww_frame_take hands the buffer over
+ * (then until agx_frame_give). */
 agx_status agx_sww_frame_wait(agx_handle h, const float** vertex, const float** centroid);
 /* As agx_sww_frame_wait, but the page-locked buffer itself (3P node values,
  * then 3N centroid values) becomes the caller's until agx_frame_give: the
  * frame is read where the device wrote it.  AGX_E_NOMEM when the callers
- * together hold 1 GiB already or no memory could be page-locked for this frame
- * (take the copy of agx_sww_frame_wait then).
- * Thread safe; the buffer outlives the scenario. */
+ * together hold 1 GiB already, no memory could be page-locked for this frame
+ * or agx_sww_frame has run since it was started (take the copy of
+ * agx_sww_frame_wait then).  As agx_sww_frame_wait it may run in a thread of
+ * its own beside the handle's other calls but agx_sww_bind and destroy, one of
+ * the two at a time; the buffer outlives the scenario.  Not for a process forked from this one: copy
+ * it before the fork. */
 agx_status agx_sww_frame_take(agx_handle h, float** frame);
 /* Gives a taken buffer back; a pointer that is not a caller's (given back
- * already, or a scenario's own) is ignored. */
+ * already, or a scenario's own) is ignored.  From any thread. */
 void agx_frame_give(float* frame);
 
 /* ---- diagnostics ------------------------------------------------------------- */

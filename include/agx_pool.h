@@ -108,7 +108,8 @@ agx_status agx_pool_sww_bind(agx_pool p, int32_t sid, int64_t P, const int32_t* 
                              const int32_t* node_slots);
 agx_status agx_pool_sww_frame_async(agx_pool p, int32_t sid, double min_storable_height, int32_t centroid_averaging);
 agx_status agx_pool_sww_frame_wait(agx_pool p, int32_t sid, const float** vertex, const float** centroid);
-/* agx_sww_frame_take for one scenario; the buffer goes back with agx_frame_give. */
+/* agx_sww_frame_take for one scenario (the pointers of a wait end with it as
+ * there); the buffer goes back with agx_frame_give. */
 agx_status agx_pool_sww_frame_take(agx_pool p, int32_t sid, float** frame);
 
 /* Evolve clock of one scenario (generic_domain.py:1715-1826): relative time,
