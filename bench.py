@@ -440,8 +440,11 @@ def measure_single(args, precision, torch, world, barrier, dist, builder):
 # lanes that did work; sm__inst_executed_pipe_fp64.sum x 32: lane slots the
 # warps occupied, idle lanes of divergent branches included) of every kernel
 # of the step (prep, then extrapolation, flux, accumulation and update of both
-# stages) on the 1.0M-triangle inflow_bumps case, divided by its cells.
+# stages) on the 1.0M-triangle inflow_bumps case, divided by its cells.  They
+# hold from min_cells on (IMUL_MIN_CELLS of agx_plain.cu): below, the step forms
+# all its products on the FP64 pipe.
 FP64_PER_CELL_STEP = {
+    "min_cells": 20000,
     "lane_ops": 3.395 + (72.78 + 58.57 + 36.01 + 27.91) + (72.78 + 58.58 + 35.02 + 26.96),
     "warp_slots": 3.469 + (77.01 + 70.57 + 37.84 + 28.75) + (77.01 + 70.57 + 36.63 + 30.67),
     "note": "ncu --metrics sm__thread_inst_executed_pipe_fp64_pred_on.sum,sm__inst_executed_pipe_fp64.sum of "
@@ -452,7 +455,10 @@ FP64_PER_CELL_STEP = {
 def fp64_roofline(cells, ms_per_step, dfma_gops):
     """The plain step against the FP64 pipe: FP64 lane operations per second
     (the instructions the step issues per cell x cells / step time) over the
-    measured DFMA rate, and the same for the lane slots the warps occupied."""
+    measured DFMA rate, and the same for the lane slots the warps occupied.
+    None for meshes whose kernels issue other counts."""
+    if cells < FP64_PER_CELL_STEP["min_cells"]:
+        return None
     sec = ms_per_step / 1e3
     ach = FP64_PER_CELL_STEP["lane_ops"] * cells / sec / 1e9
     occ = FP64_PER_CELL_STEP["warp_slots"] * cells / sec / 1e9
