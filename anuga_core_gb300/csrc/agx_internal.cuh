@@ -140,9 +140,10 @@ __host__ __device__ inline int clock_logic(Clock* c) {
 
 // The last block of a kernel to finish runs timestep_logic or clock_logic
 // itself.  Its SM's L1 may hold lines of the clock from before the other
-// blocks' atomics, so the fields these change are read past it and stored
-// back, which the thread's own later loads see; no other field changes while
-// the kernel runs.
+// blocks' atomics, so the fields these change and the two functions read are
+// read past it and stored back, which the thread's own later loads see.  The
+// update's atomics change mass_added and the cell counts too, which neither
+// function reads or writes.
 __device__ __forceinline__ void clock_refresh(Clock* c) {
   c->error = __ldcg(&c->error);
   c->bfs_acc = __ldcg(&c->bfs_acc);

@@ -564,13 +564,13 @@ __device__ __forceinline__ void flux_phase(const PoolDev& d, EdgeState* es) {
     float ew = 0.f, ex = 0.f, ey = 0.f, smax = 0.f, bfl = 0.f;
     float4 g3 = make_float4(0.f, 0.f, 0.f, 0.f), g4 = g3;
     double sw = 0.0, suh = 0.0, svh = 0.0;
-    // A cell whose three edges are dry on both sides (edge depths exactly
+    // A dry cell whose three edges are dry on both sides (edge depths exactly
     // zero; no boundary, riverwall or unstaged neighbour) has a zero flux:
     // every term the loop below would add is +0 (both Audusse depths are
     // zero, so the flux, the speed and the pressure terms vanish), so the
-    // loop and its geometry loads are skipped with the same result.
-    // Looked at only where the cell itself is dry: a wet cell's edge depths
-    // are all zero by accident at most, and the loop gives the same.
+    // loop and its geometry loads are skipped with the same result.  A wet
+    // cell goes through the loop whatever its edges: its bed slope term, g/2 of
+    // its own depth times the bed's step at each edge, is not zero.
     bool dry = valid && rk.x == 0.0f && cn.x >= 0 && cn.y >= 0 && cn.z >= 0 && !(EXT && ((cn.w >> 20) & 7));
     if (dry) {
 #pragma unroll

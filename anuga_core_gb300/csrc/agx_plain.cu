@@ -764,7 +764,6 @@ cudaError_t enqueue_saxpy(Scenario* s, cudaStream_t st, double a, double b) {
   return cudaSuccess;
 }
 
-// One full timestep (Euler, RK2 or RK3), ending with the clock kernel.
 cudaError_t enqueue_geo_transpose(Scenario* s, cudaStream_t st, const double* rows) {
   if (s->d.N == 0) return cudaSuccess;
   LAUNCH(k_geo_transpose<<<nblk(s->d.N), TPB, 0, st>>>((double*)s->d.geo, rows, s->d.N));

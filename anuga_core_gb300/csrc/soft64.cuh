@@ -265,8 +265,8 @@ SF_HD double mul(double a, double b) {
 // a / b by three digits of the quotient n / d in [1, 2) (n, d the
 // significands): each digit is the nearest integer to the FP32 quotient of the remainder's
 // leading 31 bits and d, scaled by 2^17, 2^18 and 2^19.  The FP32 relative
-// error is below 2^-21 (d's cut 2^-30, reciprocal, product and conversion 2^-22.4
-// together), so a digit is off by less than 0.5 + 2^-2 of the scaled quotient,
+// error is below 2^-21 (the quotient's 2 ulp 2^-22, two conversions and a
+// product 2^-24 each, two cuts 2^-30), so a digit is off by less than 0.5 + 2^-2 of the scaled quotient,
 // the remainders (exact in 64-bit wrap-around arithmetic) stay below d in
 // magnitude, the next digits below 2^19, and the last remainder gives the
 // floor after one correction and the sticky bit.
