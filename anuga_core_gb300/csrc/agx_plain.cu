@@ -669,9 +669,19 @@ __global__ void k_clock(Dev d, cudaGraphConditionalHandle handle, int set_cond) 
 
 // ---------------------------------------------------------------------------
 static inline int nblk(int n) { return (n + TPB - 1) / TPB; }
-// Meshes from here on take the integer products (see imul): 40,000 cells 2772
-// us a run with them and 2922 without, 396 cells the other way round; at
-// 20,000 cells a block of four warps per SM is all there is.
+// Meshes from here on take the integer products (see imul).  us a step with
+// them and without, two scenes in DE0 and DE1 (dam DE0, inflow DE0, dam DE1,
+// inflow DE1):
+//    4,900 cells   41.3/39.1   42.4/39.6   69.9/65.1   74.2/67.4
+//   14,900         43.9/43.7   43.6/40.9   75.7/73.0   78.3/72.4
+//   20,200         46.9/45.4   46.9/45.5   79.1/81.0   81.6/79.3
+//   30,300         51.8/54.8   50.2/50.3   88.8/92.9   86.5/85.7
+//   40,000         58.5/62.9   54.1/55.6  101.7/109.6  97.2/99.0
+//  160,000        137.6/154.9 119.2/129.0 249.4/282.7 214.7/236.4
+// With few warps a scheduler the longer chain of an integer product shows, with
+// many the FP64 pipe is full.  They cross between 20,000 and 30,000 cells, the
+// extrapolation first, the accumulation last; the difference there is within 4%
+// either way.
 constexpr int IMUL_MIN_CELLS = 20000;
 static inline int xblk(int n) { return (n + XCELLS - 1) / XCELLS; }
 
