@@ -3,6 +3,7 @@ library's calls replaced: over the buffer itself, given back once with the last
 array over it, or the caller's own copies where it cannot be handed over."""
 import ctypes
 import gc
+import os
 
 import numpy as np
 import pytest
@@ -54,3 +55,14 @@ def test_frame_arrays(monkeypatch, P, N, refuse):
     del part
     gc.collect()
     assert L.given == ([] if refuse else [L.buffer.ctypes.data])
+
+
+def test_a_forked_process_gives_nothing_back(monkeypatch):
+    L = _Library(6, False)
+    monkeypatch.setattr(_lib, "load", lambda: L)
+    v, c = _lib._frame_arrays(L.take, None, (None,), 1, 1)
+    here = os.getpid()
+    monkeypatch.setattr(os, "getpid", lambda: here + 1)      # its copy of the arrays goes
+    del v, c
+    gc.collect()
+    assert not L.given
