@@ -213,7 +213,7 @@ struct Scenario {
   int* node_off = nullptr;
   int* node_slot = nullptr;
   float* frame = nullptr;
-  float* frame_host = nullptr;           // page-locked copy of the last frame (null once taken)
+  float* frame_host = nullptr;           // host copy of the last frame (null once taken)
   size_t frame_bytes = 0;                // of that copy; 0: not bound for output
   bool frame_only = false;               // the device buffer has another frame: the copy stays the scenario's
   std::mutex frame_mu;                   // a frame may be waited for by a thread of its own
